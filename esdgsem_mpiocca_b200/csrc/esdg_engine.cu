@@ -34,6 +34,7 @@
 #include "esdg_analysis.cuh"
 #include "esdg_geometry.cuh"
 #include "esdg_okada.cuh"
+#include "esdg_resident.hpp"
 #include "esdg_setup.hpp"
 
 namespace esdg {
@@ -175,6 +176,8 @@ class Engine {
 
     // step graph
     cudaGraphExec_t graph = nullptr;
+    bool graph_stale = false;  // the executable graph predates the current time loop's settings
+    bool loop_ready = false;   // a time loop has been set up on this stream
     std::vector<double> gA, gB, gC;
     int gStages = 0;
 
@@ -205,6 +208,9 @@ class Engine {
 
     void release() {
         if (graph) { cudaGraphExecDestroy(graph); graph = nullptr; }
+        loop_ready = false;
+        res = ResShape{0, 0, 0, 0, 0, 0, 0};
+        res_words = nullptr;
         for (auto& e : pev)
             if (e) cudaEventDestroy(e);
         pev.clear();
@@ -432,7 +438,72 @@ class Engine {
             }
             if (r) return r;
         }
+        if ((r = setup_resident())) return r;
         built = true;
+        return 0;
+    }
+
+    // ---- chip-resident time loop (esdg_resident.cu) ----
+    // A small single mesh without artificial viscosity, manufactured source
+    // or analysis outputs runs its steps inside one cooperative kernel; the
+    // rule is that the state fits the SMs' shared memory.
+    ResShape res{0, 0, 0, 0, 0, 0, 0};
+    double* res_words = nullptr;             // exchanged words: traces, then wave-speed keys
+    unsigned long long res_epoch = 0;        // epochs used so far
+    static constexpr int RES_STEPS = 1024;   // steps per launch at most
+
+    int setup_resident() {
+        res = ResShape{0, 0, 0, 0, 0, 0, 0};
+        if (AV || conv || elem_inst || arrival || max_elev) return 0;
+        int sms = 0, coop = 0;
+        cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+        if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceGetAttribute");
+        if (!coop) return 0;
+        const bool extra = PP || PartialDry;
+        const ResShape s = resident_shape(ngl, K, sms, extra);
+        if (s.grid <= 0) return 0;
+        e = resident_setup(ngl, s, extra);
+        if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute (resident loop)");
+        int r = 0;
+        if (!res_words && (r = alloc(&res_words, ((size_t)K * 24 * ngl + 2 * (size_t)s.grid) * 2))) return r;
+        e = cudaDeviceSynchronize();  // the zero fills ran on the legacy stream
+        if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceSynchronize");
+        res = s;
+        return 0;
+    }
+
+    // A fixed element variant and the bulk-wait test hook concern the step
+    // graph's element kernels.
+    bool use_resident() const {
+        return res.grid > 0 && forced_variant < 0 && dbg_wait_limit == 0 && dbg_skip_tile == 0;
+    }
+
+    // Up to nsteps steps (at most RES_STEPS) in one launch.  *ok: false when
+    // the device refused the launch (the caller takes the step graph).
+    int launch_resident(int nsteps, bool* ok) {
+        ResArgs a;
+        std::memset(&a, 0, sizeof a);
+        a.K = K; a.ngl = ngl;
+        a.Jinv = Jinv; a.Yxi = Yxi; a.Yeta = Yeta; a.Xxi = Xxi; a.Xeta = Xeta; a.Bx = Bx; a.By = By; a.D = D;
+        a.q = q; a.gRK = gRK; a.ftab = ftab; a.side = side; a.nx = nx; a.ny = ny; a.scal = scal; a.bL = bL; a.bR = bR;
+        a.tr = reinterpret_cast<ResWord*>(res_words);
+        a.lam = reinterpret_cast<ResWord*>(res_words + (size_t)K * 48 * ngl);
+        a.epoch = res_epoch;
+        res_epoch += (unsigned long long)(nsteps + 1) * gStages;
+        a.st = st; a.c = phys();
+        for (int s = 0; s < gStages; ++s) { a.rkA[s] = gA[s]; a.rkB[s] = gB[s]; a.rkC[s] = gC[s]; }
+        a.stages = gStages; a.ssp = rkSSP; a.numflux = NumFlux; a.nsteps = nsteps;
+        a.PP = PP; a.EleSizes = EleSizes; a.GLw = GLw;
+        if (PartialDry) { a.dry_on = dry; a.B = B; a.Dc = DcFD; a.Dup = DupFD; a.Ddn = DdnFD; }
+        *ok = true;
+        const cudaError_t e = resident_launch(a, res, PP || PartialDry, stream);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            *ok = false;
+            return 0;
+        }
+        ++launches;
         return 0;
     }
 
@@ -1095,6 +1166,8 @@ class Engine {
     int capture_step_graph() {
         const long long before = launches;
         cudaGraph_t gr;
+        graph_stale = false;
+        loop_ready = true;
         cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return cuda_fail(e, "cudaStreamBeginCapture");
         ESDG_DISPATCH(ngl, launch_step);
@@ -1139,11 +1212,23 @@ class Engine {
             int r = poll_state();
             if (r) return r;
             if (st_host->done) break;
-            long long todo = chunk;
+            const bool resident = use_resident();
+            long long todo = resident ? RES_STEPS : chunk;
             if (nsteps > 0) {
                 if (done_steps >= nsteps) break;
                 todo = std::min<long long>(todo, nsteps - done_steps);
             }
+            if (resident) {
+                bool ok = false;
+                if ((r = launch_resident((int)todo, &ok))) return r;
+                if (ok) {
+                    done_steps += todo;
+                    continue;
+                }
+                res = ResShape{0, 0, 0, 0, 0, 0, 0};
+                todo = std::min<long long>(todo, chunk);
+            }
+            if ((!graph || graph_stale) && ((r = run_autotune()) || (r = capture_step_graph()))) return r;
             for (long long k = 0; k < todo; ++k) {
                 cudaError_t e = cudaGraphLaunch(graph, stream);
                 if (e != cudaSuccess) return cuda_fail(e, "cudaGraphLaunch");
@@ -1171,8 +1256,8 @@ class Engine {
         if (e != cudaSuccess) return cuda_fail(e, "state upload");
         ESDG_DISPATCH(ngl, launch_bottom);
         ESDG_DISPATCH(ngl, launch_lambda);
-        if ((r = run_autotune())) return r;
-        if ((r = capture_step_graph())) return r;
+        graph_stale = true;
+        loop_ready = true;
         if ((r = run_steps(max_steps > 0 ? max_steps : 0))) return r;
         if ((r = poll_state())) return r;
         if (t_out) *t_out = st_host->t;
@@ -1199,7 +1284,7 @@ class Engine {
     int resume(double* t_out, int* steps_out) {
         int r = check_ready();
         if (r) return r;
-        if (!graph) return fail(ESDG_E_ARG, "esdg_resume needs a previous esdg_dg_timeloop call");
+        if (!loop_ready) return fail(ESDG_E_ARG, "esdg_resume needs a previous esdg_dg_timeloop call");
         if ((r = poll_state())) return r;
         const bool finished = !(st_host->t < st_host->T) ||
                               (st_host->max_steps > 0 && st_host->steps >= st_host->max_steps) ||
@@ -1226,7 +1311,7 @@ class Engine {
     int advance(int nsteps, double T, double* t_out, int* steps_out) {
         int r = check_ready();
         if (r) return r;
-        if (!graph) return fail(ESDG_E_ARG, "esdg_advance needs a previous esdg_dg_timeloop call");
+        if (gStages <= 0) return fail(ESDG_E_ARG, "esdg_advance needs a previous esdg_dg_timeloop call");
         if ((r = poll_state())) return r;
         st_host->T = T;
         st_host->done = 0;
@@ -1238,10 +1323,23 @@ class Engine {
         st_host->max_steps = target;
         e = cudaMemcpyAsync(st, st_host, sizeof(DevState), cudaMemcpyHostToDevice, stream);
         if (e != cudaSuccess) return cuda_fail(e, "state upload");
-        for (int k = 0; k < nsteps; ++k) {
+        loop_ready = true;
+        for (int k = 0; k < nsteps;) {
+            if (use_resident()) {
+                bool ok = false;
+                const int todo = std::min(nsteps - k, (int)RES_STEPS);
+                if ((r = launch_resident(todo, &ok))) return r;
+                if (ok) {
+                    k += todo;
+                    continue;
+                }
+                res = ResShape{0, 0, 0, 0, 0, 0, 0};
+            }
+            if ((!graph || graph_stale) && ((r = run_autotune()) || (r = capture_step_graph()))) return r;
             e = cudaGraphLaunch(graph, stream);
             if (e != cudaSuccess) return cuda_fail(e, "cudaGraphLaunch");
             launches += kernels_per_step;
+            ++k;
         }
         if ((r = poll_state())) return r;
         if (t_out) *t_out = st_host->t;
@@ -1307,6 +1405,7 @@ class Engine {
         if (r) return r;
         if (gStages <= 0) return fail(ESDG_E_ARG, "profile_steps needs a previous esdg_dg_timeloop call");
         if (AV && indicator) return fail(ESDG_E_UNSUPPORTED, "profile_steps times the reference path (indicator 0)");
+        if ((r = run_autotune())) return r;
         const size_t nev = (size_t)nsteps * gStages * 3;
         while (pev.size() < nev) {
             cudaEvent_t e = nullptr;
@@ -1592,8 +1691,16 @@ int esdg_indicator_stats(esdg_deviceclass* d, unsigned long long* counts4, int r
     return d->eng.indicator_stats(counts4, reset);
 }
 
+// The resident loop needs no element kernel, so a mesh that runs in it is
+// tuned when its variants are asked for after a time loop.
+static void tune_if_asked(const esdg_deviceclass* d) {
+    esdg::Engine& E = const_cast<esdg_deviceclass*>(d)->eng;
+    if (!E.tma_tuned && E.loop_ready && E.use_resident() && cudaSetDevice(E.device) == cudaSuccess) E.run_autotune();
+}
+
 int esdg_tuned_config(const esdg_deviceclass* d, int* ctas_per_sm, int* stages, float* ms_variants3) {
     if (!d) return ESDG_E_ARG;
+    tune_if_asked(d);
     const esdg::Engine& E = d->eng;
     const int v = E.tma_variant;
     const bool node_kernel = v < esdg::TMA_VARIANTS;
@@ -1618,6 +1725,7 @@ static int element_variants(const esdg::Engine& E, int* chosen, int* count, floa
 int esdg_element_variants(const esdg_deviceclass* d, int* chosen, int* count, float* ms, int* ctas_per_sm,
                           int cap) {
     if (!d) return ESDG_E_ARG;
+    tune_if_asked(d);
     return element_variants(d->eng, chosen, count, ms, ctas_per_sm, cap);
 }
 
@@ -1640,6 +1748,7 @@ int esdg_set_stream(esdg_deviceclass* d, void* cuda_stream) {
     esdg::Engine& E = d->eng;
     E.stream = cuda_stream ? static_cast<cudaStream_t>(cuda_stream) : E.own_stream;
     if (E.graph) { cudaGraphExecDestroy(E.graph); E.graph = nullptr; }
+    E.loop_ready = false;
     return ESDG_OK;
 }
 
@@ -1668,11 +1777,6 @@ int esdg_debug_bulk_wait_test(esdg_deviceclass* d, long long wait_limit_cycles, 
 int esdg_advance(esdg_deviceclass* d, int nsteps, double T, double* t_out, int* steps_out) {
     ESDG_GUARD(d);
     if (nsteps < 0) return d->eng.fail(ESDG_E_ARG, "nsteps < 0");
-    if (!d->eng.graph) {
-        if (d->eng.gStages <= 0) return d->eng.fail(ESDG_E_ARG, "esdg_advance needs a previous esdg_dg_timeloop call");
-        int r = d->eng.capture_step_graph();
-        if (r) return r;
-    }
     return d->eng.advance(nsteps, T, t_out, steps_out);
 }
 

@@ -992,7 +992,7 @@ __global__ void __launch_bounds__(ElemShape<NGL>::THREADS) k_lambda(int K, const
 // Step bookkeeping per instance (src/deviceclass.cpp:897-930 and :1130):
 // dt from the CFL and viscous limits, done flag when t >= T or the step cap
 // is reached.
-__global__ void k_step_begin(int I, DevState* st, int ngl, int AV) {
+static __global__ void k_step_begin(int I, DevState* st, int ngl, int AV) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= I) return;
     DevState& s = st[k];
@@ -1015,7 +1015,7 @@ __global__ void k_step_begin(int I, DevState* st, int ngl, int AV) {
     s.visc_key = 0ull;
 }
 
-__global__ void k_step_end(int I, DevState* st) {
+static __global__ void k_step_end(int I, DevState* st) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= I) return;
     DevState& s = st[k];
