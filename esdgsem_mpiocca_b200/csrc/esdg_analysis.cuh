@@ -27,6 +27,8 @@ __global__ void __launch_bounds__(256) k_analysis(long nodes, const double* __re
                                                   const double* __restrict__ B, const DevState* __restrict__ st,
                                                   double h_zero, double* __restrict__ arrival,
                                                   double* __restrict__ max_elev) {
+    pdl_release();
+    pdl_wait();
     const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nodes || st[0].done) return;
     const long e = k / N2;

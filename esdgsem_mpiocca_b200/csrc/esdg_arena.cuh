@@ -99,6 +99,7 @@ class Arena : public Engine {
             (r = h2d(Vinv, B.VdmInv.data(), B.VdmInv.size(), "Vinv")) ||
             (r = h2d(GLw, B.wGL.data(), B.wGL.size(), "GLw")))
             return r;
+        if (AV_) k_build_nbr<<<(K + 255) / 256, 256, 0, stream>>>(0, K, side, ftab, nbr);
         Vinv_h = B.VdmInv;
         Dfd_h = B.D;
         copied = true;
@@ -177,6 +178,7 @@ class Arena : public Engine {
             return r;
         }
         cudaMemsetAsync(gRK + eo * n2 * 3, 0, nn * 3 * sizeof(double), stream);
+        if (AV) cudaMemsetAsync(act + eo, 0, (size_t)K_ * sizeof(int), stream);
         // step state, owner map, bathymetry traces, initial wave speed
         DevState s0;
         std::memset(&s0, 0, sizeof s0);

@@ -19,10 +19,12 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <mutex>
 #include <new>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/esdg_b200.h"
@@ -128,7 +130,7 @@ class Engine {
     double *Bx = nullptr, *By = nullptr, *B = nullptr, *X = nullptr, *Y = nullptr;
     double *D = nullptr, *Dstrong = nullptr, *Dhat = nullptr, *Vinv = nullptr, *GLw = nullptr, *EleSizes = nullptr;
     double *nx = nullptr, *ny = nullptr, *scal = nullptr, *bL = nullptr, *bR = nullptr, *SP = nullptr;
-    double *SGX = nullptr, *SGY = nullptr, *SPV = nullptr, *GX = nullptr, *GY = nullptr, *VP = nullptr;
+    double *SGX = nullptr, *SGY = nullptr, *GX = nullptr, *GY = nullptr, *VP = nullptr;
     int *EdgeData = nullptr;
     int4 *ftab = nullptr, *side = nullptr;
     // analysis outputs per node (initDeviceVariables' CalcArrivalTimes and
@@ -139,10 +141,9 @@ class Engine {
     int* elem_inst = nullptr;     // null: one instance
     int I = 1;                    // step-state entries (instances, arena: + one retired slot)
 
-    // Troubled-cell indicator of the artificial-viscosity path: 0 the modal
-    // sensor and the viscous terms on every element (the reference's path);
-    // 1 the modal sensor with the active set (viscous terms only on flagged
-    // elements, same numbers); 2 the learned indicator with the active set
+    // Troubled-cell indicator of the artificial-viscosity path: 0 and 1 the
+    // modal sensor (the reference's path; the viscous terms run on the active
+    // set, exactly zero elsewhere); 2 the learned indicator with the active set
     // (one fused pass where the degree allows, N = 3); 3 the same decisions
     // by three passes (features, network, sensor) at every degree.
     int indicator = 0;
@@ -171,7 +172,6 @@ class Engine {
     double *DcFD = nullptr, *DupFD = nullptr, *DdnFD = nullptr;
     bool pd_copied = false;
     int list_grid = 0;                        // persistent grid of the list kernels
-    int face_list_grid = 0;                   // grid of the viscous face kernel over the listed elements' faces
     int ind_grid[3] = {1, 1, 1};              // persistent grids of the indicator (modal, learned, fused)
 
     // step graph
@@ -239,6 +239,8 @@ class Engine {
         c.sigmaMax = sigma_max;
         c.ZeroTOL = std::pow(10.0, -5);
         c.sensor_skip = std::isfinite(sigma_min) ? std::pow(10.0, sigma_min) * (1.0 - 1e-12) : 0.0;
+        c.sensor_full = std::isfinite(sigma_max) && sigma_min <= sigma_max ? std::pow(10.0, sigma_max) * (1.0 + 1e-12)
+                                                                          : std::numeric_limits<double>::infinity();
         c.ES = ES;
         return c;
     }
@@ -278,8 +280,9 @@ class Engine {
                 return r;
         }
         if (AV) {
-            if ((r = alloc(&SGX, nf * 2)) || (r = alloc(&SGY, nf * 2)) || (r = alloc(&SPV, nf * 2)) ||
-                (r = alloc(&GX, nn * 2)) || (r = alloc(&GY, nn * 2)) || (r = alloc(&VP, (size_t)K)))
+            if ((r = alloc(&SGX, nf * 2)) || (r = alloc(&SGY, nf * 2)) ||
+                (r = alloc(&GX, nn * 2)) || (r = alloc(&GY, nn * 2)) || (r = alloc(&VP, (size_t)K)) ||
+                (r = alloc(&act, (size_t)K + 1)) || (r = alloc(&alist, (size_t)K)) || (r = alloc(&nbr, (size_t)K)))
                 return r;
         }
         if (ArrivalTimes_) {
@@ -290,6 +293,8 @@ class Engine {
         }
         if (MaxElevation_ && (r = alloc(&max_elev, nn))) return r;  // from 0, as the reference's calloc
         if ((r = alloc(&st, (size_t)I))) return r;
+        const ResShape rs = resident_candidate();
+        if (rs.grid > 0 && (r = alloc(&res_words, ((size_t)K * 24 * ngl + 2 * (size_t)rs.grid) * 2))) return r;
         cudaError_t e = cudaMallocHost(&st_host, sizeof(DevState));
         if (e != cudaSuccess) return cuda_fail(e, "cudaMallocHost");
         // the zero fills ran on the legacy stream; order them before any
@@ -363,6 +368,7 @@ class Engine {
         if (Qt_h && (r = h2d(Qt, Qt_h, nd, "Qt"))) return r;
         if (PP_ && (r = h2d(GLw, GLw_h, (size_t)ngl, "GLw"))) return r;
         if (!PP_ && GLw_h && (r = h2d(GLw, GLw_h, (size_t)ngl, "GLw"))) return r;
+        if (AV) k_build_nbr<<<(K + 255) / 256, 256, 0, stream>>>(0, K, side, ftab, nbr);
         cudaError_t e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return cuda_fail(e, "copyDeviceVariables");
         Vinv_h.assign(Vinv_h_, Vinv_h_ + n2);
@@ -452,24 +458,26 @@ class Engine {
     unsigned long long res_epoch = 0;        // epochs used so far
     static constexpr int RES_STEPS = 1024;   // steps per launch at most
 
+    // The launch shape, zeros where the step graph has to run: artificial
+    // viscosity, analysis outputs, an arena (I > 1), or too many elements.
+    ResShape resident_candidate() const {
+        int sms = 0, coop = 0;
+        if (AV || arrival || max_elev || I > 1 ||
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+            cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop)
+            return ResShape{0, 0, 0, 0, 0, 0, 0};
+        return resident_shape(ngl, K, sms, PP || PartialDry);
+    }
+
     int setup_resident() {
         res = ResShape{0, 0, 0, 0, 0, 0, 0};
-        if (AV || conv || elem_inst || arrival || max_elev) return 0;
-        int sms = 0, coop = 0;
-        cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceGetAttribute");
-        if (!coop) return 0;
+        if (conv) return 0;
         const bool extra = PP || PartialDry;
-        const ResShape s = resident_shape(ngl, K, sms, extra);
+        const ResShape s = resident_candidate();
         if (s.grid <= 0) return 0;
-        e = resident_setup(ngl, s, extra);
+        const cudaError_t e = resident_setup(ngl, s, extra);
         if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute (resident loop)");
-        int r = 0;
-        if (!res_words && (r = alloc(&res_words, ((size_t)K * 24 * ngl + 2 * (size_t)s.grid) * 2))) return r;
-        e = cudaDeviceSynchronize();  // the zero fills ran on the legacy stream
-        if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceSynchronize");
-        res = s;
+        if (res_words) res = s;
         return 0;
     }
 
@@ -508,6 +516,34 @@ class Engine {
     }
 
     // ---- kernel launchers (dispatch on ngl) ----
+    // Launch of one of the step's kernels (each begins with pdl_wait): in a
+    // step it may start while the kernel before it drains, which hides its
+    // launch and prologue.  chained: the operation before it on the stream
+    // is such a kernel too (a copy or a memset is waited for in full).
+    // Small meshes only: the launches are what a step of theirs waits for
+    // (576 elements of N = 4 with viscosity: 109.5 -> 99.8 us a step; 480,000
+    // nodes of N = 6: 2.8 % faster), while on large ones the next kernel's
+    // early blocks only take room (512x512, N = 4: no gain; 1.6 million nodes
+    // with viscosity everywhere: 8 % slower).
+    bool pdl_on = false, chained = false;
+    bool pdl_pays() const { return (long long)K * ngl * ngl <= (AV ? 150000 : 600000); }
+
+    template <class... P, class... A>
+    void launch(void (*k)(P...), int grid, int block, size_t smem, A&&... args) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3((unsigned)block);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = pdl_on && chained ? 1 : 0;
+        cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
+        chained = true;
+    }
+
     // Blocks of a face-node (or element-warp) kernel over n threads: one pass
     // for a single mesh; for an arena a resident grid that strides over the
     // live extent (the capacity can be far above the live part).
@@ -523,31 +559,20 @@ class Engine {
     template <int NGL, bool STRIDE>
     void launch_face_k(const FaceArgs& a, bool av_grad, int blocks) {
         if (av_grad) {
-            if (NumFlux == 0) k_face_flux<NGL, 0, true, STRIDE><<<blocks, 256, 0, stream>>>(a);
-            else if (NumFlux == 2) k_face_flux<NGL, 2, true, STRIDE><<<blocks, 256, 0, stream>>>(a);
-            else k_face_flux<NGL, 3, true, STRIDE><<<blocks, 256, 0, stream>>>(a);
+            if (NumFlux == 0) launch(k_face_flux<NGL, 0, true, STRIDE>, blocks, 256, 0, a);
+            else if (NumFlux == 2) launch(k_face_flux<NGL, 2, true, STRIDE>, blocks, 256, 0, a);
+            else launch(k_face_flux<NGL, 3, true, STRIDE>, blocks, 256, 0, a);
         } else {
-            if (NumFlux == 0) k_face_flux<NGL, 0, false, STRIDE><<<blocks, 256, 0, stream>>>(a);
-            else if (NumFlux == 2) k_face_flux<NGL, 2, false, STRIDE><<<blocks, 256, 0, stream>>>(a);
-            else k_face_flux<NGL, 3, false, STRIDE><<<blocks, 256, 0, stream>>>(a);
+            if (NumFlux == 0) launch(k_face_flux<NGL, 0, false, STRIDE>, blocks, 256, 0, a);
+            else if (NumFlux == 2) launch(k_face_flux<NGL, 2, false, STRIDE>, blocks, 256, 0, a);
+            else launch(k_face_flux<NGL, 3, false, STRIDE>, blocks, 256, 0, a);
         }
-    }
-
-    // viscous face flux, one-shot for a single mesh, strided for an arena
-    template <int NGL>
-    void launch_face_visc(long n, const int* actp, const int* ext) {
-        if (elem_inst)
-            k_face_visc<NGL, true><<<face_blocks(n), 256, 0, stream>>>(F, ftab, nx, ny, scal, GX, GY, VP, SPV,
-                                                                      elem_inst, st, geomFace, actp, ext);
-        else
-            k_face_visc<NGL, false><<<face_blocks(n), 256, 0, stream>>>(F, ftab, nx, ny, scal, GX, GY, VP, SPV,
-                                                                       elem_inst, st, geomFace, actp, ext);
     }
 
     template <int NGL>
     int launch_face(bool av_grad) {
         FaceArgs a{F, ftab, q, nx, ny, scal, bL, bR, SP, SGX, SGY, elem_inst, st, phys()};
-        a.act = (AV && indicator) ? act : nullptr;
+        a.act = act;
         a.extent = extent;
         if (conv) { a.conv = 1; a.tfrac = stage_tfrac; a.X = X; a.Y = Y; }
         const long n = (long)F * NGL;
@@ -562,7 +587,7 @@ class Engine {
         ElemArgs a;
         a.K = K; a.Jinv = Jinv; a.Yxi = Yxi; a.Yeta = Yeta; a.Xxi = Xxi; a.Xeta = Xeta; a.Bx = Bx; a.By = By;
         a.B = B; a.D = D; a.Dhat = Dhat; a.Dstrong = Dstrong; a.Vinv = Vinv; a.SP = SP; a.SGX = SGX; a.SGY = SGY;
-        a.SPV = SPV; a.side = side; a.q = q; a.gRK = gRK; a.Qt = Qt; a.Qtmp = Qtmp; a.GX = GX; a.GY = GY; a.VP = VP;
+        a.side = side; a.ftab = ftab; a.nx = nx; a.ny = ny; a.scal = scal; a.q = q; a.gRK = gRK; a.Qt = Qt; a.Qtmp = Qtmp; a.GX = GX; a.GY = GY; a.VP = VP;
         a.elem_inst = elem_inst; a.st = st; a.rkA = A; a.rkB = Bc; a.rkC = C; a.mode = mode; a.lam = lam;
         a.c = phys(); a.extent = extent;
         if (PartialDry) {
@@ -682,11 +707,11 @@ class Engine {
         const int ntiles = (K + P::NE - 1) / P::NE;
         const int gen = elem_gen(ea);
         if (gen == 0)
-            k_element_pair<NGL, pair_min_blocks(V), 0><<<tma_grid[PAIR_FIRST + V], P::THREADS, P::SMEM, stream>>>(ea, ntiles);
+            launch(k_element_pair<NGL, pair_min_blocks(V), 0>, tma_grid[PAIR_FIRST + V], P::THREADS, P::SMEM, ea, ntiles);
         else if (gen == 2)
-            k_element_pair<NGL, pair_min_blocks(V), 2><<<tma_grid[PAIR_FIRST + V], P::THREADS, P::SMEM, stream>>>(ea, ntiles);
+            launch(k_element_pair<NGL, pair_min_blocks(V), 2>, tma_grid[PAIR_FIRST + V], P::THREADS, P::SMEM, ea, ntiles);
         else
-            k_element_pair<NGL, pair_min_blocks(V), 1><<<tma_grid[PAIR_FIRST + V], P::THREADS, P::SMEM, stream>>>(ea, ntiles);
+            launch(k_element_pair<NGL, pair_min_blocks(V), 1>, tma_grid[PAIR_FIRST + V], P::THREADS, P::SMEM, ea, ntiles);
     }
 
     template <int NGL>
@@ -716,11 +741,11 @@ class Engine {
         // the instance with the branches this step does not need compiled out
         const int gen = elem_gen(ea);
         if (gen == 0)
-            k_element_tma<NGL, tma_min_blocks(V), tma_stages(V), 0><<<tma_grid[V], T::THREADS, T::SMEM, stream>>>(ea, ntiles);
+            launch(k_element_tma<NGL, tma_min_blocks(V), tma_stages(V), 0>, tma_grid[V], T::THREADS, T::SMEM, ea, ntiles);
         else if (gen == 2)
-            k_element_tma<NGL, tma_min_blocks(V), tma_stages(V), 2><<<tma_grid[V], T::THREADS, T::SMEM, stream>>>(ea, ntiles);
+            launch(k_element_tma<NGL, tma_min_blocks(V), tma_stages(V), 2>, tma_grid[V], T::THREADS, T::SMEM, ea, ntiles);
         else
-            k_element_tma<NGL, tma_min_blocks(V), tma_stages(V), 1><<<tma_grid[V], T::THREADS, T::SMEM, stream>>>(ea, ntiles);
+            launch(k_element_tma<NGL, tma_min_blocks(V), tma_stages(V), 1>, tma_grid[V], T::THREADS, T::SMEM, ea, ntiles);
     }
 
     template <int NGL, int R>
@@ -731,8 +756,7 @@ class Engine {
             DLine<NGL> dm;
             for (int i = 0; i < NGL * NGL; ++i) dm.v[i] = Dfd_h[i];
             const int ntiles = (K + NE - 1) / NE;
-            k_element_rows<NGL, NE, 2, row_min_blocks(R)>
-                <<<tma_grid[TMA_VARIANTS + R], T::THREADS, T::SMEM, stream>>>(ea, dm, ntiles);
+            launch(k_element_rows<NGL, NE, 2, row_min_blocks(R)>, tma_grid[TMA_VARIANTS + R], T::THREADS, T::SMEM, ea, dm, ntiles);
         }
     }
 
@@ -753,7 +777,7 @@ class Engine {
             launch_tma<NGL>(ea, tma_variant);
         } else {
             using S = ElemShape<NGL>;
-            k_element<NGL><<<(K + S::NE - 1) / S::NE, S::THREADS, 0, stream>>>(ea);
+            launch(k_element<NGL>, (K + S::NE - 1) / S::NE, S::THREADS, 0, ea);
         }
         ++launches;
     }
@@ -801,6 +825,7 @@ class Engine {
         ElemArgs ea = elem_args(rkSSP ? 1 : 0, have ? gA[0] : 0.0, have ? gB[0] : 1.0, have ? gC[0] : 0.0, 0);
         ea.q = tq;
         ea.gRK = tg;
+        if (AV) { ea.act = act; ea.alist = alist; ea.acount = act + K; }  // the instance that a viscous stage runs
         for (int v = 0; v < ELEM_VARIANTS; ++v)
             if (tma_grid[v] > 0) launch_tma<NGL>(ea, v);  // first-launch costs
         for (int r = 0; r < REPS; ++r)
@@ -837,48 +862,46 @@ class Engine {
         return 0;
     }
 
+    // Element kernel, then the viscous terms of the elements it listed.
+    // clear: the flags are taken back for the next sensor pass.
+    template <int NGL>
+    void launch_viscous_stage(ElemArgs ea, bool clear) {
+        using S = ElemShape<NGL>;
+        ea.act = act; ea.alist = alist; ea.acount = act + K;
+        ea.clear_act = clear;
+        launch_elem_plain<NGL>(ea);
+        launch(k_grad_list<NGL>, list_grid, S::THREADS, 0, ea);
+        launch(k_viscous_list<NGL>, list_grid, S::THREADS, 0, ea);
+        launches += 2;
+    }
+
     template <int NGL>
     void launch_stage(int mode, double A, double Bc, double C, bool last, bool shock_stage) {
         using S = ElemShape<NGL>;
         const int eb = (K + S::NE - 1) / S::NE;
         const int lam_in_elem = (last && !PP) ? 1 : 0;
         launch_find_dry<NGL>();
-        if (AV && indicator) {
-            // active set: indicator (stages > 0; stage 0's runs before the
-            // step's dt), plain element kernel (flagged elements only write
-            // Qt and are listed), then gradient, viscous face flux and
-            // viscous update over the list
+        if (AV) {
+            // the sensor (stages > 0; stage 0's runs before the step's dt)
+            // flags the active set; the plain element kernel updates the
+            // other elements, writes Qt of the flagged ones and lists them;
+            // gradient, viscous face flux and viscous update over the list
             if (shock_stage) {
                 if (ind_every_stage || indicator < 2) launch_indicator<NGL>(0);
-                else cudaMemsetAsync(act + K, 0, sizeof(int), stream);  // the step's flags, a new list
+                else {
+                    cudaMemsetAsync(act + K, 0, sizeof(int), stream);  // the step's flags, a new list
+                    chained = false;
+                }
             }
             launch_face<NGL>(true);
-            ElemArgs ea = elem_args(mode, A, Bc, C, lam_in_elem);
-            ea.act = act; ea.alist = alist; ea.acount = act + K;
-            launch_elem_plain<NGL>(ea);
-            k_grad_list<NGL><<<list_grid, S::THREADS, 0, stream>>>(ea);
-            // the viscous face fluxes of the listed elements' faces only
-            k_face_visc_list<NGL><<<face_list_grid, 256, 0, stream>>>(side, ftab, nx, ny, scal, GX, GY, VP, SPV,
-                                                                      elem_inst, st, geomFace, act, alist, act + K);
-            k_element_av2<NGL><<<list_grid, S::THREADS, 0, stream>>>(ea);
-            launches += 3;
-        } else if (!AV) {
+            launch_viscous_stage<NGL>(elem_args(mode, A, Bc, C, lam_in_elem),
+                                      last || mode == 2 || ind_every_stage || indicator < 2);
+        } else {
             launch_face<NGL>(false);
             launch_elem_plain<NGL>(elem_args(mode, A, Bc, C, lam_in_elem));
-        } else {
-            // the reference path: the sensor (same arithmetic as okl/ShockCapturing,
-            // one entry of the modal transform per thread) then the viscous
-            // terms on every element
-            if (shock_stage) launch_indicator<NGL>(0);
-            launch_face<NGL>(true);
-            k_element_av1<NGL><<<eb, S::THREADS, 0, stream>>>(elem_args(2, A, Bc, C, 0));
-            const long n = (long)F * NGL;
-            launch_face_visc<NGL>(n, nullptr, nullptr);
-            k_element_av2<NGL><<<eb, S::THREADS, 0, stream>>>(elem_args(mode, A, Bc, C, lam_in_elem));
-            launches += 3;
         }
         if (PP && mode != 2) {
-            k_pospres<NGL><<<eb, S::THREADS, 0, stream>>>(K, EleSizes, GLw, Jinv, q, elem_inst, st, last ? 1 : 0,
+            launch(k_pospres<NGL>, eb, S::THREADS, 0, K, EleSizes, GLw, Jinv, q, elem_inst, st, last ? 1 : 0,
                                                           phys());
             ++launches;
         }
@@ -894,9 +917,8 @@ class Engine {
 
     template <int NGL>
     void launch_indicator(int stage0) {
-        if (indicator) cudaMemsetAsync(act, 0, (size_t)(K + 1) * sizeof(int), stream);
         IndArgs ia;
-        ia.K = K; ia.q = q; ia.B = B; ia.Vinv = Vinv; ia.VP = VP; ia.act = indicator ? act : nullptr; ia.nbr = nbr;
+        ia.K = K; ia.q = q; ia.B = B; ia.Vinv = Vinv; ia.VP = VP; ia.act = act; ia.acount = act + K; ia.nbr = nbr;
         ia.elem_inst = elem_inst; ia.st = st; ia.c = phys(); ia.stage0 = stage0;
         ia.P = mlpP; ia.Pb = mlpPb; ia.L = mlp_layout(NGL); ia.margin = ind_margin;
         ia.emin = ind_emin; ia.emax = ind_emax; ia.stats = ind_stats; ia.extent = extent;
@@ -908,7 +930,7 @@ class Engine {
                 // features, network and sensor fallback in one pass
                 using FS = FusedShape<NGL>;
                 const int ftiles = (K + FS::NE - 1) / FS::NE;
-                k_indicator_fused<NGL><<<std::min(ftiles, ind_grid[2]), FS::THREADS, 0, stream>>>(ia, ftiles);
+                launch(k_indicator_fused<NGL>, std::min(ftiles, ind_grid[2]), FS::THREADS, 0, ia, ftiles);
                 ++launches;
             }
         } else if (indicator >= 2) {
@@ -917,16 +939,20 @@ class Engine {
                 // features, forward pass, then the sensor where unsure
                 constexpr int KP = mlp_kp(NGL);
                 if constexpr ((32 % (NGL * NGL)) == 0)
-                    k_ind_features<NGL><<<std::min(ntiles, ind_grid[0]), S::THREADS, 0, stream>>>(ia, ntiles);
+                    launch(k_ind_features<NGL>, std::min(ntiles, ind_grid[0]), S::THREADS, 0, ia, ntiles);
                 else
-                    k_ind_features_warp<NGL><<<face_blocks((long)K * 32), 256, 0, stream>>>(ia);
-                k_mlp_forward<KP><<<mlp_grid, 128, MlpSmem<KP>::fwd_bytes(4), stream>>>(K, indX, mlpP, mlpPb, ind_y,
+                    launch(k_ind_features_warp<NGL>, face_blocks((long)K * 32), 256, 0, ia);
+                launch(k_mlp_forward<KP>, mlp_grid, 128, MlpSmem<KP>::fwd_bytes(4), K, indX, mlpP, mlpPb, ind_y,
                                                                                  ia.L, extent);
-                k_indicator<NGL, true><<<std::min(ntiles, ind_grid[1]), S::THREADS, 0, stream>>>(ia, ntiles);
+                launch(k_indicator<NGL>, std::min(ntiles, ind_grid[1]), S::THREADS, 0, ia, ntiles);
                 launches += 3;
             }
         } else {
-            k_indicator<NGL, false><<<std::min(ntiles, ind_grid[0]), S::THREADS, 0, stream>>>(ia, ntiles);
+            using SS = SensorShape<NGL>;
+            SensorV<NGL> V;
+            for (int i = 0; i < NGL * NGL; ++i) V.v[i] = Vinv_h[i];
+            const int per = SS::EPW * SS::WARPS;
+            launch(k_sensor<NGL>, std::min((K + per - 1) / per, ind_grid[0]), SS::WARPS * 32, 0, ia, V);
             ++launches;
         }
     }
@@ -935,19 +961,15 @@ class Engine {
     int setup_indicator() {
         using S = ElemShape<NGL>;
         int a2 = 0, gr = 0, sms = 0;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a2, k_element_av2<NGL>, S::THREADS, 0);
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a2, k_viscous_list<NGL>, S::THREADS, 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&gr, k_grad_list<NGL>, S::THREADS, 0);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         if (e != cudaSuccess) return cuda_fail(e, "occupancy (list kernels)");
         list_grid = std::max(1, std::min(std::max(1, std::min(a2, gr)) * sms, (K + S::NE - 1) / S::NE));
-        int fv = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fv, k_face_visc_list<NGL>, 256, 0);
-        if (e != cudaSuccess) return cuda_fail(e, "occupancy (viscous face list)");
-        face_list_grid = std::max(1, std::min(std::max(1, fv) * sms, (int)(((long)K * 4 * NGL + 255) / 256)));
         int o0 = 0, o1 = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o0, k_indicator<NGL, false>, IndShape<NGL>::THREADS, 0);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o0, k_sensor<NGL>, SensorShape<NGL>::WARPS * 32, 0);
         if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o1, k_indicator<NGL, true>, IndShape<NGL>::THREADS, 0);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o1, k_indicator<NGL>, IndShape<NGL>::THREADS, 0);
         if (e != cudaSuccess) return cuda_fail(e, "occupancy (indicator)");
         ind_grid[0] = std::max(1, o0) * sms;
         ind_grid[1] = std::max(1, o1) * sms;
@@ -999,14 +1021,11 @@ class Engine {
             if (!(margin >= 0.0f)) return fail(ESDG_E_ARG, "learned indicator: margin must be >= 0");
         }
         int r = 0;
-        if (mode > 0 && !act) {
-            if ((r = alloc(&act, (size_t)K + 1)) || (r = alloc(&alist, (size_t)K)) || (r = alloc(&ind_stats, 4)) ||
-                (r = alloc(&nbr, (size_t)K)))
-                return r;
+        if (mode > 0 && !ind_stats) {
+            if ((r = alloc(&ind_stats, 4))) return r;
             // the zero fills ran on the legacy stream
             cudaError_t e = cudaDeviceSynchronize();
             if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceSynchronize");
-            k_build_nbr<<<(K + 255) / 256, 256, 0, stream>>>(0, K, side, ftab, nbr);
         }
         if (mode >= 2) {
             const int n = mlp_layout(ngl).total;
@@ -1065,28 +1084,32 @@ class Engine {
     void launch_analysis() {
         if (!arrival && !max_elev) return;
         const long nodes = (long)K * NGL * NGL;
-        k_analysis<NGL * NGL><<<(unsigned)((nodes + 255) / 256), 256, 0, stream>>>(nodes, q, B, st, h0, arrival,
+        launch(k_analysis<NGL * NGL>, (unsigned)((nodes + 255) / 256), 256, 0, nodes, q, B, st, h0, arrival,
                                                                                    max_elev);
         ++launches;
     }
 
     template <int NGL>
     void launch_step() {
+        pdl_on = pdl_pays();
+        chained = false;
         if (AV) launch_indicator<NGL>(1);
-        k_step_begin<<<(I + 127) / 128, 128, 0, stream>>>(I, st, ngl, AV);
+        launch(k_step_begin, (I + 127) / 128, 128, 0, I, st, ngl, AV);
         ++launches;
         if (rkSSP) {
             // o_Qtmp.copyFrom(o_q) (src/deviceclass.cpp:933-936)
             cudaMemcpyAsync(Qtmp, q, (size_t)K * ngl * ngl * 3 * sizeof(double), cudaMemcpyDeviceToDevice, stream);
+            chained = false;
         }
         for (int s = 0; s < gStages; ++s) {
             stage_tfrac = stage_time_fraction(s);
             launch_stage<NGL>(rkSSP ? 1 : 0, gA[s], gB[s], gC[s], s == gStages - 1, s > 0);
         }
         stage_tfrac = 0.0;
-        k_step_end<<<(I + 127) / 128, 128, 0, stream>>>(I, st);
+        launch(k_step_end, (I + 127) / 128, 128, 0, I, st);
         ++launches;
         launch_analysis<NGL>();
+        pdl_on = false;
     }
 
 #define ESDG_DISPATCH(NGLV, CALL)                 \
@@ -1133,7 +1156,7 @@ class Engine {
     template <int NGL>
     void launch_find_dry() {
         if (!PartialDry) return;
-        k_find_dry<NGL><<<(K + 255) / 256, 256, 0, stream>>>(K, q, dry, PosPresTOL);
+        launch(k_find_dry<NGL>, (K + 255) / 256, 256, 0, K, q, dry, PosPresTOL);
         ++launches;
     }
 
@@ -1254,6 +1277,8 @@ class Engine {
         *st_host = s0;
         cudaError_t e = cudaMemcpyAsync(st, st_host, sizeof(DevState), cudaMemcpyHostToDevice, stream);
         if (e != cudaSuccess) return cuda_fail(e, "state upload");
+        if (AV && (e = cudaMemsetAsync(act, 0, ((size_t)K + 1) * sizeof(int), stream)) != cudaSuccess)
+            return cuda_fail(e, "active set");
         ESDG_DISPATCH(ngl, launch_bottom);
         ESDG_DISPATCH(ngl, launch_lambda);
         graph_stale = true;
@@ -1374,19 +1399,12 @@ class Engine {
             stage_tfrac = stage_time_fraction(s);
             launch_find_dry<NGL>();
             cudaEvent_t* ev = pe + 3 * s;
+            if (AV && s > 0) launch_indicator<NGL>(0);
             cudaEventRecord(ev[0], stream);
             launch_face<NGL>(AV != 0);
             cudaEventRecord(ev[1], stream);
-            if (!AV) {
-                launch_elem_plain<NGL>(elem_args(mode, gA[s], gB[s], gC[s], lam_in_elem));
-            } else {
-                if (s > 0) launch_indicator<NGL>(0);
-                k_element_av1<NGL><<<eb, S::THREADS, 0, stream>>>(elem_args(2, gA[s], gB[s], gC[s], 0));
-                const long n = (long)F * NGL;
-                launch_face_visc<NGL>(n, nullptr, nullptr);
-                k_element_av2<NGL><<<eb, S::THREADS, 0, stream>>>(elem_args(mode, gA[s], gB[s], gC[s], lam_in_elem));
-                launches += 3;
-            }
+            if (!AV) launch_elem_plain<NGL>(elem_args(mode, gA[s], gB[s], gC[s], lam_in_elem));
+            else launch_viscous_stage<NGL>(elem_args(mode, gA[s], gB[s], gC[s], lam_in_elem), true);
             cudaEventRecord(ev[2], stream);
             if (PP) {
                 k_pospres<NGL><<<eb, S::THREADS, 0, stream>>>(K, EleSizes, GLw, Jinv, q, elem_inst, st, last ? 1 : 0,
@@ -2245,7 +2263,8 @@ extern "C" int esdg_compute_rhs_noalloc(int N, int K, int F, int NumFlux, int ES
     PhysConst c;
     c.g = g_const; c.half_g = 0.5 * g_const; c.fourth_g = 0.25 * g_const;
     c.geomFace = 1.0 / (2.0 / (N * (N + 1.0)));
-    c.PosPresTOL = PosPresTOL; c.eps0 = 0; c.sigmaMin = 0; c.sigmaMax = 0; c.ZeroTOL = std::pow(10.0, -5); c.sensor_skip = 0.0; c.ES = ES;
+    c.PosPresTOL = PosPresTOL; c.eps0 = 0; c.sigmaMin = 0; c.sigmaMax = 0; c.ZeroTOL = std::pow(10.0, -5); c.sensor_skip = 0.0;
+    c.sensor_full = std::numeric_limits<double>::infinity(); c.ES = ES;
     switch (ngl) {
         case 2: noalloc_launch<2>(K, F, NumFlux, c, q, Jinv, y_xi, y_eta, x_xi, x_eta, Bx, By, Dmat, nx, ny, scal, base, L, Qt, s); break;
         case 3: noalloc_launch<3>(K, F, NumFlux, c, q, Jinv, y_xi, y_eta, x_xi, x_eta, Bx, By, Dmat, nx, ny, scal, base, L, Qt, s); break;

@@ -3,16 +3,15 @@
 // on every element).
 //
 // Per element e it writes the artificial viscosity VP[e] and, where
-// VP[e] > 0 and an active set is kept (act non-null), flags e and its face
-// neighbours in act[] (zeroed before the launch).  Without act it is the
-// reference path's sensor pass.  The viscous terms of an element vanish exactly unless it or a
+// VP[e] > 0, flags e and its face neighbours in act[] (k_viscous_list takes
+// the flags back), and it resets the list's length.  The viscous terms of an element vanish exactly unless it or a
 // neighbour has VP > 0 (the face viscosity is max(VP_L, VP_R), the volume
 // term is VP_e times the gradient), so the stage's viscous kernels run on
 // the flagged elements only and give the same numbers as on all of them.
 //
-// LEARNED = false: the modal sensor (the arithmetic of
+// k_sensor: the modal sensor (the arithmetic of
 // okl/ShockCapturing/ShockCapturing.okl:17-234) on every element.
-// LEARNED = true: the MLP (esdg_mlp.cuh) predicts sigma; its answer is
+// Learned (k_indicator, k_indicator_fused): the MLP (esdg_mlp.cuh) predicts sigma; its answer is
 // used only where it is confident -- sigma_hat < sigma_min - margin gives
 // VP = 0, sigma_hat > sigma_max + margin gives VP = eps0 -- and the modal
 // sensor decides every other element: the ramp band, elements failing the
@@ -20,11 +19,10 @@
 // elements whose modal energy may be near the sensor's absolute ZeroTOL
 // threshold (bounded from the nodal energy by emin/emax).
 //
-// Layout: like the element kernels, NE elements per block and one thread
-// per node.  The modal transform runs one entry per thread (the same
-// arithmetic as the serial loops), the order-dependent sums one thread per
-// element.  For the network, one warp runs the block's (<= 16) feature rows
-// through the tensor cores.
+// Layout of k_indicator: like the element kernels, NE elements per block and
+// one thread per node.  The modal transform runs one entry per thread (the
+// same arithmetic as the serial loops), the order-dependent sums one thread
+// per element.
 #pragma once
 
 #include "esdg_mlp.cuh"
@@ -38,6 +36,7 @@ struct IndArgs {
     const double* __restrict__ Vinv;
     double* __restrict__ VP;
     int* act;
+    int* acount;                   // length of the active set's list, reset for the stage
     const int4* __restrict__ nbr;  // face neighbours (k_build_nbr)
     const int* __restrict__ extent = nullptr;  // live extent ([0] elements), as in FaceArgs
     const int* __restrict__ elem_inst;
@@ -104,6 +103,7 @@ __global__ void __launch_bounds__(IndShape<NGL>::THREADS) k_ind_features(IndArgs
     using S = IndShape<NGL>;
     constexpr int N2 = S::N2, NE = S::NE, KP = mlp_kp(NGL);
     static_assert((32 % N2) == 0, "element = aligned lane group");
+    pdl_wait();
     if (a.extent) ntiles = min(ntiles, (a.extent[0] + NE - 1) / NE);
     const int tid = threadIdx.x;
     const int el = tid / N2, nd = tid % N2;
@@ -266,6 +266,7 @@ __device__ __forceinline__ void ind_features_warp_elem(const IndArgs& a, int e) 
 // with the one-shot grid of a single mesh, a resident grid for an arena).
 template <int NGL>
 __global__ void __launch_bounds__(256) k_ind_features_warp(IndArgs a) {
+    pdl_wait();
     const int lim = a.extent ? min(a.K, a.extent[0]) : a.K;
     for (int e = blockIdx.x * 8 + (threadIdx.x >> 5); e < lim; e += gridDim.x * 8)  // warp-uniform
         ind_features_warp_elem<NGL>(a, e);
@@ -299,15 +300,179 @@ __device__ __forceinline__ IndLoad ind_load(const IndArgs& a, int t) {
         L.h = a.q[(long)e * 3 * N2 + nd];
         L.b = a.B[(long)e * N2 + nd];
         L.ins = inst_of(a.elem_inst, e);
-        if (nd == 0 && a.act) L.nb = a.nbr[e];
+        if (nd == 0) L.nb = a.nbr[e];
     }
     return L;
 }
 
-// The sensor pass (the learned variant after k_ind_features and
-// k_mlp_forward).  Persistent: each block walks tiles of NE elements, the
+// The modal sensor on every element: n threads per element (32 / n elements
+// a warp), thread j with the element's row j (eta = j) in registers.
+//
+// The transform's first product needs one row only, so thread j forms column
+// j of M1 from its registers and the matrix (kernel parameters: constant
+// bank operands); the second needs a row of M1, exchanged once through
+// shared memory.  That is 2n + 2n^2/n loads and stores per row where one
+// entry per thread takes 4n per node, and no block barrier.  Every entry's
+// sums keep the order of sensor_m1 / sensor_w, and where the any-order
+// screen cannot settle the element the reference-order tail runs on the
+// entries in shared memory: the same values bit for bit.
+//
+// 11.1 us at 1.6 million nodes of N = 4 (33.8 with one entry per thread and
+// the serial sums on every element), 2.4 TB/s of the 16 B per node it reads.
+template <int NGL>
+struct SensorV {
+    double v[NGL * NGL];
+};
+template <int NGL>
+struct SensorShape {
+    static constexpr int N2 = NGL * NGL;
+    static constexpr int EPW = 32 / NGL;                   // elements per warp
+    static constexpr int S = NGL | 1;                      // row stride of an element's matrix
+    static constexpr int GS = NGL * S;                     // element stride: n = 4 free of bank conflicts
+    static constexpr int WARPS = 8;
+};
+
+template <int NGL>
+__global__ void __launch_bounds__(SensorShape<NGL>::WARPS * 32) k_sensor(IndArgs a, const SensorV<NGL> V) {
+    using L = SensorShape<NGL>;
+    constexpr int N2 = L::N2, N = NGL - 1, EPW = L::EPW, S = L::S;
+    __shared__ double sM[L::WARPS][EPW * L::GS];
+    __shared__ double sZ[L::WARPS][EPW * 4 * NGL];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int grp = min(lane / NGL, EPW - 1), j = lane % NGL;
+    const bool mine = lane < EPW * NGL;
+    const int lim = a.extent ? min(a.K, a.extent[0]) : a.K;
+    double* M = sM[warp] + grp * L::GS;
+    double* Z = sZ[warp] + grp * 4 * NGL;
+    unsigned cnt = 0, cntv = 0;
+    pdl_wait();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.acount = 0;
+    for (int t = blockIdx.x * L::WARPS + warp; t * EPW < lim; t += gridDim.x * L::WARPS) {
+        if ((t + gridDim.x * L::WARPS) * EPW >= lim) pdl_release();  // the warp's last elements
+        const int e = t * EPW + grp;
+        const bool in = mine && e < lim;
+        double m[NGL];
+        if (in) {
+            const double* hp = a.q + (long)e * 3 * N2 + j * NGL;
+            const double* bp = a.B + (long)e * N2 + j * NGL;
+            if constexpr (NGL % 2 == 0) {  // rows start on 16 bytes
+#pragma unroll
+                for (int l = 0; l < NGL; l += 2) {
+                    const double2 h = *reinterpret_cast<const double2*>(hp + l);
+                    const double2 b = *reinterpret_cast<const double2*>(bp + l);
+                    m[l] = b.x + h.x;
+                    m[l + 1] = b.y + h.y;
+                }
+            } else {
+#pragma unroll
+                for (int l = 0; l < NGL; ++l) m[l] = bp[l] + hp[l];
+            }
+        } else {
+#pragma unroll
+            for (int l = 0; l < NGL; ++l) m[l] = 0.0;
+        }
+        const int ins = in ? inst_of(a.elem_inst, e) : 0;
+        const bool live = in && !a.st[ins].done;
+        if (mine) {
+#pragma unroll
+            for (int i = 0; i < NGL; ++i) {
+                double acc = 0.0;
+#pragma unroll
+                for (int l = 0; l < NGL; ++l) acc += V.v[i * NGL + l] * m[l];
+                M[i * S + j] = acc;
+            }
+        }
+        __syncwarp();
+        double w[NGL];
+        {
+            double r[NGL];
+#pragma unroll
+            for (int l = 0; l < NGL; ++l) r[l] = M[j * S + l];
+#pragma unroll
+            for (int k = 0; k < NGL; ++k) {
+                double acc = 0.0;
+#pragma unroll
+                for (int l = 0; l < NGL; ++l) acc += r[l] * V.v[k * NGL + l];
+                w[k] = acc;
+            }
+        }
+        // Screen: energy ratios from sums in any order differ from the
+        // reference-order ones by rounding only; far below the 10^sigma_min
+        // bound the sensor is exactly zero, far above the 10^sigma_max one
+        // exactly eps0.
+        double z1 = 0.0, z2 = 0.0, n1 = 0.0, n2 = 0.0;
+#pragma unroll
+        for (int k = 0; k < NGL; ++k) {
+            const double w2 = w[k] * w[k];
+            n1 += w2;
+            if (j == N || k == N) z1 += w2;
+            else {
+                n2 += w2;
+                if (j == N - 1 || k == N - 1) z2 += w2;
+            }
+        }
+        if (mine) {
+            Z[j] = z1; Z[NGL + j] = z2; Z[2 * NGL + j] = n1; Z[3 * NGL + j] = n2;
+        }
+        __syncwarp();
+        double Z1 = 0.0, Z2 = 0.0, N1 = 0.0, N2s = 0.0;
+        if (j == 0) {
+#pragma unroll
+            for (int k = 0; k < NGL; ++k) {
+                Z1 += Z[k]; Z2 += Z[NGL + k]; N1 += Z[2 * NGL + k]; N2s += Z[3 * NGL + k];
+            }
+        }
+        const double thr = a.c.sensor_skip * (1.0 - 1e-6), top = a.c.sensor_full * (1.0 + 1e-6);
+        const bool sure = N1 > a.c.ZeroTOL * (1.0 + 1e-6);
+        // (a NaN compares false everywhere)
+        const bool clear = (sure && Z1 < thr * N1 && Z2 < thr * N2s) || N1 < a.c.ZeroTOL * (1.0 - 1e-6);
+        const bool full = sure && N2s > 0.0 && (Z1 > top * N1 || Z2 > top * N2s) && isfinite(N1);
+        const bool lead = live && j == 0;
+        const bool tail = lead && !clear && !full;
+        if (__any_sync(0xffffffffu, tail)) {  // M's rows are read: the entries take their place
+            if (mine) {
+#pragma unroll
+                for (int k = 0; k < NGL; ++k) M[j * S + k] = w[k];
+            }
+            __syncwarp();
+        }
+        double v = 0.0;
+        if (lead && !clear) v = full ? a.c.eps0 : sensor_tail<NGL, S>(a.c, M);
+        if (a.stage0) {  // the step's largest viscosity: one atomic a warp for a single mesh
+            const unsigned long long key = v > 0.0 ? dbl_key(v) : 0ull;
+            if (a.elem_inst) {
+                if (key) atomicMax(&a.st[ins].visc_key, key);
+            } else {
+                const unsigned hi = (unsigned)(key >> 32), mhi = __reduce_max_sync(0xffffffffu, hi);
+                const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? (unsigned)key : 0u);
+                if (lane == 0 && (mhi | mlo)) atomicMax(&a.st[0].visc_key, ((unsigned long long)mhi << 32) | mlo);
+            }
+        }
+        if (lead) {
+            a.VP[e] = v;
+            cnt += 1;
+            // NaN flags too: its viscous path runs as it would everywhere
+            if (!(v <= 0.0)) {
+                mark_active(a.act, e, a.nbr[e]);
+                cntv += 1;
+            }
+        }
+        __syncwarp();  // the warp's shared rows are rewritten next tile
+    }
+    if (a.stats) {
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        cntv = __reduce_add_sync(0xffffffffu, cntv);
+        if (lane == 0) {
+            if (cnt) atomicAdd(&a.stats[2], (unsigned long long)cnt);
+            if (cntv) atomicAdd(&a.stats[3], (unsigned long long)cntv);
+        }
+    }
+}
+
+// The decision and the sensor where it is needed, after k_ind_features and
+// k_mlp_forward.  Persistent: each block walks tiles of NE elements, the
 // next tiles' loads in flight while the current one is processed.
-template <int NGL, bool LEARNED>
+template <int NGL>
 __global__ void __launch_bounds__(IndShape<NGL>::THREADS, 3) k_indicator(IndArgs a, int ntiles) {
     using S = IndShape<NGL>;
     constexpr int N2 = S::N2, NE = S::NE;
@@ -317,12 +482,14 @@ __global__ void __launch_bounds__(IndShape<NGL>::THREADS, 3) k_indicator(IndArgs
     __shared__ double sV[N2];
     __shared__ double seta[NE * N2], sM[NE * N2], sW[NE * N2];
     __shared__ int need[NE];
-    __shared__ int verdict[NE];  // learned: 0 zero, 1 eps0 (when need == 0)
+    __shared__ int verdict[NE];  // 0 zero, 1 eps0 (when need == 0)
 
     const int tid = threadIdx.x;
     const int el = tid / N2, nd = tid % N2;
     const int s = el * N2 + nd;
     if (tid < N2) sV[tid] = a.Vinv[tid];
+    pdl_wait();
+    if (blockIdx.x == 0 && tid == 0) *a.acount = 0;
     unsigned long long cnt[4] = {0, 0, 0, 0};
     constexpr int PF = 2;  // tiles of loads in flight
     int t = blockIdx.x;
@@ -345,7 +512,7 @@ __global__ void __launch_bounds__(IndShape<NGL>::THREADS, 3) k_indicator(IndArgs
         seta[s] = cur.b + cur.h;
         if (nd == 0) {
             int nm = 1, vd = 0;
-            if (LEARNED && live) {
+            if (live) {
                 const double sig = (double)a.y[e] + (double)a.seta[e];
                 const double nodal = a.energy[e];
                 nm = learned_needs_modal(a, sig, nodal, a.ok[e]);
@@ -354,9 +521,8 @@ __global__ void __launch_bounds__(IndShape<NGL>::THREADS, 3) k_indicator(IndArgs
             need[el] = nm;
             verdict[el] = vd;
         }
-        // the modal transform where the sensor decides (every element
-        // without the network)
-        const bool any = LEARNED ? __syncthreads_or(live && nd == 0 && need[el]) : (__syncthreads(), true);
+        // the modal transform where the sensor decides
+        const bool any = __syncthreads_or(live && nd == 0 && need[el]);
         bool clear = false;
         if (any) {
             const int i = nd / NGL, j = nd % NGL;  // entry (i, j) of M1 and w
@@ -400,7 +566,7 @@ __global__ void __launch_bounds__(IndShape<NGL>::THREADS, 3) k_indicator(IndArgs
             a.VP[e] = v;
             if (a.stage0 && v > 0.0) atomicMax(&a.st[cur.ins].visc_key, dbl_key(v));
             // NaN flags too: its viscous path runs as on the full path
-            if (a.act && !(v <= 0.0)) mark_active(a.act, e, cur.nb);
+            if (!(v <= 0.0)) mark_active(a.act, e, cur.nb);
             cnt[kind] += 1;
             if (!(v <= 0.0)) cnt[3] += 1;
         }
@@ -423,7 +589,7 @@ __global__ void __launch_bounds__(IndShape<NGL>::THREADS, 3) k_indicator(IndArgs
 // the rest the element's lanes, so every per-element sum -- means, nodal
 // energy, deviations -- and the positivity check are those of the feature
 // pass bit for bit.  The modal transform, its screen (n = 4, as in
-// k_indicator<4, true>) and the tail follow k_indicator<NGL, true> entry by
+// k_indicator<4>) and the tail follow k_indicator<NGL> entry by
 // entry.  Each warp runs the network on its own 32 / (W/4) feature rows
 // (mlp_warp_forward_rows: a 16-row MMA tile with every row repeated, each
 // row's dot products those of k_mlp_forward).  Inside the tile loop no warp
@@ -481,6 +647,8 @@ __global__ void __launch_bounds__(FusedShape<NGL>::THREADS, 3) k_indicator_fused
         sP32[2 * MLP_H + i] = a.P[a.L.w3 + i];
     }
     if (tid == 0) sP32[3 * MLP_H] = a.P[a.L.b3];
+    pdl_wait();
+    if (blockIdx.x == 0 && tid == 0) *a.acount = 0;
     __syncthreads();  // the only block barrier: V and the network staged
     double* se = seta + el * ES;
     double* sm = sM + el * ES;
@@ -515,7 +683,7 @@ __global__ void __launch_bounds__(FusedShape<NGL>::THREADS, 3) k_indicator_fused
         }
         if (inb) {
             ins = inst_of(a.elem_inst, e);
-            if (j == 0 && a.act) nb = a.nbr[e];
+            if (j == 0) nb = a.nbr[e];
         }
         const bool live = inb && !a.st[ins].done;
         // ---- features (the feature pass) ----
@@ -584,7 +752,7 @@ __global__ void __launch_bounds__(FusedShape<NGL>::THREADS, 3) k_indicator_fused
         // ---- network (k_mlp_forward) on the warp's rows ----
         const float yw = mlp_warp_forward_rows<KP, EPW, XS, XS, W2S>(sX + warp * EPW * XS, sW1, sW2, sP32);
         const float y = __shfl_sync(0xffffffffu, yw, 4 * (lane / TPE));  // row r's output sits in quad r
-        // ---- decision and modal fallback (k_indicator<NGL, true>) ----
+        // ---- decision and modal fallback (k_indicator<NGL>) ----
         int nm = 1, vd = 0;
         if (live) {
             const double sig = (double)y + (double)s_eta;
@@ -638,7 +806,7 @@ __global__ void __launch_bounds__(FusedShape<NGL>::THREADS, 3) k_indicator_fused
             }
             a.VP[e] = v;
             if (a.stage0 && v > 0.0) atomicMax(&a.st[ins].visc_key, dbl_key(v));
-            if (a.act && !(v <= 0.0)) mark_active(a.act, e, nb);
+            if (!(v <= 0.0)) mark_active(a.act, e, nb);
             cnt[kind] += 1;
             if (!(v <= 0.0)) cnt[3] += 1;
         }

@@ -24,6 +24,8 @@
 #include <cuda_bf16.h>
 #include <mma.h>
 
+#include "esdg_pdl.cuh"
+
 namespace esdg {
 
 constexpr int MLP_H = 32;
@@ -459,6 +461,7 @@ __global__ void __launch_bounds__(128) k_mlp_forward(int M, const __nv_bfloat16*
                                                      const float* __restrict__ P,
                                                      const __nv_bfloat16* __restrict__ Pb, float* __restrict__ y,
                                                      MlpLayout L, const int* __restrict__ Mlive = nullptr) {
+    pdl_wait();
     if (Mlive) M = min(M, *Mlive);  // rows past a live extent are skipped
     using S = MlpSmem<KP>;
     constexpr int VPR = KP / 8;        // 16-byte vectors per row

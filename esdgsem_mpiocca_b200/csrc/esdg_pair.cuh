@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(PairShape<NGL>::THREADS, MINB) k_element_pair(
     }
     if (tid == 0)
         for (int k = 0; k < ST; ++k) mbar_init(&bar[k], 1);
+    pdl_wait();
     __syncthreads();
     if (tid == 0)
         for (int k = 0; k < ST; ++k) {
@@ -61,6 +62,7 @@ __global__ void __launch_bounds__(PairShape<NGL>::THREADS, MINB) k_element_pair(
         }
     int it = 0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
+        if (t + gridDim.x >= ntiles) pdl_release();  // the CTA's last tile
         const int sidx = it % ST;
         const unsigned parity = (unsigned)((it / ST) & 1);
         double* sb = stage + sidx * P::STAGE_DOUBLES;
@@ -87,6 +89,7 @@ __global__ void __launch_bounds__(PairShape<NGL>::THREADS, MINB) k_element_pair(
             to_list[k] = GEN != 0 && active[k] && a.act && a.act[e[k]] != 0;
             dt[k] = (active[k] && a.mode != 2) ? a.st[ins[k]].dt : 0.0;
         }
+        if (GEN != 0 && a.act && tid < 32) list_tile(a, e0, NE);
         // every thread waits for the tile; a copy that never lands makes the
         // whole CTA leave together (uniform decision) with an error status
         // for the host instead of hanging
@@ -178,7 +181,6 @@ __global__ void __launch_bounds__(PairShape<NGL>::THREADS, MINB) k_element_pair(
             const long qid = (long)e[k] * 3 * N2 + nd;
             if (a.mode == 2 || to_list[k]) {
                 a.Qt[qid] = r0; a.Qt[qid + N2] = r1; a.Qt[qid + 2 * N2] = r2;
-                if (to_list[k] && nd == 0) a.alist[atomicAdd(a.acount, 1)] = e[k];
             } else {
                 const double o0 = s2[qs], o1 = s2[qs + N2], o2 = s2[qs + 2 * N2];
                 double q0, q1, q2;

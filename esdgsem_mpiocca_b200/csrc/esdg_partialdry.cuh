@@ -17,6 +17,8 @@ namespace esdg {
 template <int NGL>
 __global__ void k_find_dry(int K, const double* __restrict__ q, int* __restrict__ dry, double tol) {
     constexpr int N2 = NGL * NGL;
+    pdl_release();
+    pdl_wait();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= K) return;
     const double* h = q + (long)e * 3 * N2;

@@ -6,6 +6,8 @@
 
 #include <cuda_runtime.h>
 
+#include "esdg_pdl.cuh"
+
 namespace esdg {
 
 struct PhysConst {
@@ -14,6 +16,10 @@ struct PhysConst {
     // energy ratio below which log10(ratio) < sigmaMin holds with margin
     // (10^sigmaMin (1 - 1e-12)): the sensor returns 0 without log10/sin
     double sensor_skip;
+    // energy ratio above which log10(ratio) > sigmaMax holds with margin
+    // (10^sigmaMax (1 + 1e-12); +inf where that decides nothing): the sensor
+    // returns eps0 without log10/sin
+    double sensor_full;
     int ES;
 };
 

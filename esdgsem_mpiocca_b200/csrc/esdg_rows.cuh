@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(RowShape<NGL, NE, ST>::THREADS, MINB)
     const int el = worker ? tid % NE : 0;
     if (tid == 0)
         for (int k = 0; k < ST; ++k) mbar_init(&bar[k], 1);
+    pdl_wait();
     __syncthreads();
     if (tid == 0)
         for (int k = 0; k < ST; ++k) {
@@ -191,6 +192,7 @@ __global__ void __launch_bounds__(RowShape<NGL, NE, ST>::THREADS, MINB)
     const double g = a.c.g;
     int it = 0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
+        if (t + gridDim.x >= ntiles) pdl_release();  // the CTA's last tile
         const int sidx = it % ST;
         const unsigned parity = (unsigned)((it / ST) & 1);
         double* sb = stage + sidx * S::STAGE_DOUBLES;
@@ -211,6 +213,7 @@ __global__ void __launch_bounds__(RowShape<NGL, NE, ST>::THREADS, MINB)
         const bool active = inb && !a.st[ins].done;
         const bool to_list = active && a.act && a.act[e] != 0;
         const double dt = (active && a.mode != 2) ? a.st[ins].dt : 0.0;
+        if (a.act && tid < 32) list_tile(a, e0, NE);
         // a copy that never lands makes the whole CTA leave together
         // (uniform decision) with an error status for the host
         const bool landed = mbar_wait_bounded(&bar[sidx], parity, a.wait_limit);
@@ -326,7 +329,6 @@ __global__ void __launch_bounds__(RowShape<NGL, NE, ST>::THREADS, MINB)
                     }
                 }
             }
-            if (to_list && ln == 0) a.alist[atomicAdd(a.acount, 1)] = e;
         }
         if (a.lam) warp_lambda<S::THREADS>(lam, active && !to_list, ins, a.st);
         if (bulk) fence_proxy_async_smem();  // shared-memory writes before the bulk store reads them

@@ -213,6 +213,7 @@ __global__ void __launch_bounds__(TmaShape<NGL>::THREADS, MINB) k_element_tma(El
     if (tid < N2) sD[tid] = a.D[tid];
     if (tid == 0)
         for (int k = 0; k < ST; ++k) mbar_init(&bar[k], 1);
+    pdl_wait();
     __syncthreads();
     if (tid == 0)
         for (int k = 0; k < ST; ++k) {
@@ -221,6 +222,7 @@ __global__ void __launch_bounds__(TmaShape<NGL>::THREADS, MINB) k_element_tma(El
         }
     int it = 0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
+        if (t + gridDim.x >= ntiles) pdl_release();  // the CTA's last tile
         const int sidx = it % ST;
         const unsigned parity = (unsigned)((it / ST) & 1);
         double* sb = stage + sidx * S::STAGE_DOUBLES;
@@ -240,6 +242,7 @@ __global__ void __launch_bounds__(TmaShape<NGL>::THREADS, MINB) k_element_tma(El
         const bool active = inb && !a.st[ins].done;
         const bool to_list = GEN != 0 && active && a.act && a.act[e] != 0;
         const double dt = (active && a.mode != 2) ? a.st[ins].dt : 0.0;
+        if (GEN != 0 && a.act && tid < 32) list_tile(a, e0, NE);
         // every thread waits for the tile; a copy that never lands makes the
         // whole CTA leave together (uniform decision) with an error status
         // for the host instead of hanging
@@ -323,7 +326,6 @@ __global__ void __launch_bounds__(TmaShape<NGL>::THREADS, MINB) k_element_tma(El
             const long qid = (long)e * 3 * N2 + nd;
             if (a.mode == 2 || to_list) {
                 a.Qt[qid] = r0; a.Qt[qid + N2] = r1; a.Qt[qid + 2 * N2] = r2;
-                if (to_list && nd == 0) a.alist[atomicAdd(a.acount, 1)] = e;
             } else {
                 const double o0 = s2[qs], o1 = s2[qs + N2], o2 = s2[qs + 2 * N2];
                 double q0, q1, q2;
