@@ -55,89 +55,101 @@ __host__ __device__ inline MlpLayout mlp_layout(int ngl) {
 
 // Modal sensor value sigma of one element: log10 of the larger of the two
 // energy ratios (okl/ShockCapturing/ShockCapturing.okl:131-204), -inf when
-// the modal energy n1 is below ZeroTOL (then *tiny is set).  m = nodal
-// (h + b) [eta][xi].
+// the modal energy n1 is below ZeroTOL (then *tiny is set).  By a warp: m =
+// nodal (h + b) [eta][xi], V, and room for the two products in shared memory;
+// an entry per lane, and the four order-dependent sums on a lane each, in the
+// reference's order.  Valid on lane 0.
 template <int NGL>
-__device__ double sensor_sigma(double ZeroTOL, const double* m, const double* V, bool* tiny) {
-    constexpr int N = NGL - 1;
-    double M1[NGL * NGL], w[NGL * NGL];
-    for (int i = 0; i < NGL; ++i)
-        for (int j = 0; j < NGL; ++j) {
-            double acc = 0.0;
-            for (int l = 0; l < NGL; ++l) acc += V[i * NGL + l] * m[j * NGL + l];
-            M1[i * NGL + j] = acc;
-        }
-    for (int i = 0; i < NGL; ++i)
-        for (int j = 0; j < NGL; ++j) {
-            double acc = 0.0;
-            for (int l = 0; l < NGL; ++l) acc += M1[i * NGL + l] * V[j * NGL + l];
-            w[i * NGL + j] = acc;
-        }
-    double z1 = 0, n1 = 0, z2 = 0, n2s = 0;
-    for (int i = 0; i < N; ++i) z1 += w[i * NGL + N] * w[i * NGL + N] + w[N * NGL + i] * w[N * NGL + i];
-    z1 += w[N * NGL + N] * w[N * NGL + N];
-    for (int i = 0; i < N - 1; ++i)
-        z2 += w[i * NGL + N - 1] * w[i * NGL + N - 1] + w[(N - 1) * NGL + i] * w[(N - 1) * NGL + i];
-    z2 += w[(N - 1) * NGL + N - 1] * w[(N - 1) * NGL + N - 1];
-    for (int i = 0; i < NGL; ++i)
-        for (int j = 0; j < NGL; ++j) n1 += w[i * NGL + j] * w[i * NGL + j];
-    for (int i = 0; i < N; ++i)
-        for (int j = 0; j < N; ++j) n2s += w[i * NGL + j] * w[i * NGL + j];
+__device__ __forceinline__ double sensor_sigma(double ZeroTOL, const double* m, const double* V, double* M1, double* w,
+                                               bool* tiny) {
+    constexpr int N = NGL - 1, N2 = NGL * NGL;
+    const int lane = threadIdx.x & 31;
+    for (int p = lane; p < N2; p += 32) {
+        const int i = p / NGL, j = p % NGL;
+        double acc = 0.0;
+        for (int l = 0; l < NGL; ++l) acc += V[i * NGL + l] * m[j * NGL + l];
+        M1[p] = acc;
+    }
+    __syncwarp();
+    for (int p = lane; p < N2; p += 32) {
+        const int i = p / NGL, j = p % NGL;
+        double acc = 0.0;
+        for (int l = 0; l < NGL; ++l) acc += M1[i * NGL + l] * V[j * NGL + l];
+        w[p] = acc;
+    }
+    __syncwarp();
+    double s = 0.0;
+    if (lane < 2) {  // z1 and z2: the two highest modes' rows and columns
+        const int n = N - lane;
+        for (int i = 0; i < n; ++i) s += w[i * NGL + n] * w[i * NGL + n] + w[n * NGL + i] * w[n * NGL + i];
+        s += w[n * NGL + n] * w[n * NGL + n];
+    } else if (lane < 4) {  // n1 and n2: all modes, without the highest
+        const int n = lane == 2 ? NGL : N;
+        for (int i = 0; i < n; ++i)
+            for (int j = 0; j < n; ++j) s += w[i * NGL + j] * w[i * NGL + j];
+    }
+    const double z1 = s, z2 = __shfl_sync(0xffffffffu, s, 1);
+    const double n1 = __shfl_sync(0xffffffffu, s, 2), n2s = __shfl_sync(0xffffffffu, s, 3);
     const double t1 = (n1 < ZeroTOL) ? 0.0 : z1 / n1;
     const double t2 = (n1 < ZeroTOL) ? 0.0 : z2 / n2s;
     *tiny = n1 < ZeroTOL;
     return log10((t1 < t2) ? t2 : t1);
 }
 
-// Normalisation of one field over an element's nodes held by a warp
-// (node p = lane + 32 k): mean, RMS of the deviation, and s.
-template <int NGL>
-__device__ __forceinline__ void mlp_field_stats(const double (&v)[(NGL * NGL + 31) / 32], double& mean, double& rms,
-                                                double& s) {
-    constexpr int N2 = NGL * NGL, R = (N2 + 31) / 32;
-    const int lane = threadIdx.x & 31;
-    double a = 0.0;
-#pragma unroll
-    for (int k = 0; k < R; ++k)
-        if (lane + 32 * k < N2) a += v[k];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
-    mean = a / N2;
-    double d2 = 0.0;
-#pragma unroll
-    for (int k = 0; k < R; ++k)
-        if (lane + 32 * k < N2) d2 += (v[k] - mean) * (v[k] - mean);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) d2 += __shfl_xor_sync(0xffffffffu, d2, off);
-    rms = sqrt(d2 / N2);
-    const double tot = mean * mean + rms * rms;
-    s = (tot > 0.0 && rms > 0.0) ? fmax(log10(rms * rms / tot), MLP_S_MIN) : MLP_S_MIN;
-}
-
 // Writes one element's feature row (bf16, KP columns) from the warp's
-// register copy of the element; returns s_eta (all lanes).
+// register copy of the element (node p = lane + 32 k): mean, RMS of the
+// deviation and s of the three fields, their butterflies side by side, and
+// one log10 pass (lanes 0, 1, 2: a field each).  Returns s_eta on lane 0.
 template <int NGL>
 __device__ __forceinline__ double mlp_feature_row(const double (&v)[3][(NGL * NGL + 31) / 32],
                                                   __nv_bfloat16* __restrict__ xr) {
     constexpr int N2 = NGL * NGL, R = (N2 + 31) / 32, KP = mlp_kp(NGL);
     const int lane = threadIdx.x & 31;
-    double s_eta = 0.0;
+    double mean[3], rms[3];
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
-        double mean, rms, s;
-        mlp_field_stats<NGL>(v[f], mean, rms, s);
+        mean[f] = 0.0;
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+            if (lane + 32 * k < N2) mean[f] += v[f][k];
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+        for (int f = 0; f < 3; ++f) mean[f] += __shfl_xor_sync(0xffffffffu, mean[f], off);
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+        mean[f] = mean[f] / N2;
+        rms[f] = 0.0;
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+            if (lane + 32 * k < N2) rms[f] += (v[f][k] - mean[f]) * (v[f][k] - mean[f]);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+        for (int f = 0; f < 3; ++f) rms[f] += __shfl_xor_sync(0xffffffffu, rms[f], off);
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+        rms[f] = sqrt(rms[f] / N2);
         // a deviation at rounding level (constant field) is not a shape
-        const double inv = (rms > MLP_REL_FLAT * fabs(mean) && rms > 0.0) ? 1.0 / rms : 0.0;
+        const double inv = (rms[f] > MLP_REL_FLAT * fabs(mean[f]) && rms[f] > 0.0) ? 1.0 / rms[f] : 0.0;
 #pragma unroll
         for (int k = 0; k < R; ++k) {
             const int p = lane + 32 * k;
-            if (p < N2) xr[f * N2 + p] = __float2bfloat16((float)((v[f][k] - mean) * inv));
+            if (p < N2) xr[f * N2 + p] = __float2bfloat16((float)((v[f][k] - mean[f]) * inv));
         }
-        if (lane == 0) xr[3 * N2 + f] = __float2bfloat16((float)(0.25 * s));
-        if (f == 0) s_eta = s;
+    }
+    double s = MLP_S_MIN;
+    if (lane < 3) {
+        const double m = lane == 0 ? mean[0] : (lane == 1 ? mean[1] : mean[2]);
+        const double r = lane == 0 ? rms[0] : (lane == 1 ? rms[1] : rms[2]);
+        const double tot = m * m + r * r;
+        if (tot > 0.0 && r > 0.0) s = fmax(log10(r * r / tot), MLP_S_MIN);
+        xr[3 * N2 + lane] = __float2bfloat16((float)(0.25 * s));
     }
     for (int p = 3 * N2 + 3 + lane; p < KP; p += 32) xr[p] = __float2bfloat16(0.0f);
-    return s_eta;
+    return s;
 }
 
 // Feature rows of every element, and optionally the training target
@@ -151,7 +163,7 @@ __global__ void __launch_bounds__(256) k_mlp_features(int K, const double* __res
                                                       float* __restrict__ seta) {
     constexpr int N2 = NGL * NGL, R = (N2 + 31) / 32, KP = mlp_kp(NGL);
     __shared__ double sV[N2];
-    __shared__ double se[8][N2];
+    __shared__ double se[8][N2], sM1[8][N2], sW[8][N2];
     const int w = threadIdx.x / 32, lane = threadIdx.x % 32;
     if (threadIdx.x < N2) sV[threadIdx.x] = Vinv[threadIdx.x];
     __syncthreads();
@@ -173,9 +185,9 @@ __global__ void __launch_bounds__(256) k_mlp_features(int K, const double* __res
     const double s_eta = mlp_feature_row<NGL>(v, X + (long)e * KP);
     if (tgt) {
         __syncwarp();
+        bool tiny = false;
+        const double sg = sensor_sigma<NGL>(ZeroTOL, se[w], sV, sM1[w], sW[w], &tiny);
         if (lane == 0) {
-            bool tiny = false;
-            const double sg = sensor_sigma<NGL>(ZeroTOL, se[w], sV, &tiny);
             const double c = fmin(fmax(sg, MLP_S_MIN), 0.0);  // -inf -> -12
             tgt[e] = tiny ? __int_as_float(0x7fc00000) : (float)(c - s_eta);
             if (seta) seta[e] = (float)s_eta;
@@ -187,13 +199,23 @@ __global__ void __launch_bounds__(256) k_mlp_features(int K, const double* __res
 
 using namespace nvcuda;
 
-// One warp's forward pass on 16 rows held in shared memory (ld = KP):
+// Row strides of the backward kernel's shared matrices (bf16 rows of KP and
+// 32 columns, float rows of 32): eight bf16 or four floats past the row, so
+// that the fragment loads of eight rows and the row walks of sixteen lanes
+// fall on different banks.
+template <int KP>
+struct MlpPad {
+    static constexpr int X = KP + 8, B = MLP_H + 8, Z = MLP_H + 4;
+};
+
+// One warp's forward pass on 16 rows held in shared memory (strides MlpPad):
 // Z1 = X W1^T + b1, A1 = relu(Z1) (bf16), Z2 = A1 W2^T + b2 (float, left
-// in z), y = relu(Z2) . w3 + b3 into y16[0..15].
+// in z), y = relu(Z2) . w3 + b3 into y16[0..15].  b1, b2: the lane's entries.
 template <int KP>
 __device__ __forceinline__ void mlp_warp_forward(const __nv_bfloat16* Xrows, const __nv_bfloat16* W1b,
-                                                 const __nv_bfloat16* W2b, const float* __restrict__ P,
-                                                 const MlpLayout& L, __nv_bfloat16* a1b, float* z, float* y16) {
+                                                 const __nv_bfloat16* W2b, const float* __restrict__ sw3, float b1,
+                                                 float b2, float b3, __nv_bfloat16* a1b, float* z, float* y16) {
+    using S = MlpPad<KP>;
     const int lane = threadIdx.x & 31;
     wmma::fragment<wmma::accumulator, 16, 16, 16, float> acc[2];
     wmma::fragment<wmma::matrix_a, 16, 16, 16, __nv_bfloat16, wmma::row_major> fa;
@@ -202,37 +224,40 @@ __device__ __forceinline__ void mlp_warp_forward(const __nv_bfloat16* Xrows, con
     for (int n = 0; n < 2; ++n) wmma::fill_fragment(acc[n], 0.0f);
 #pragma unroll
     for (int k = 0; k < KP / 16; ++k) {
-        wmma::load_matrix_sync(fa, Xrows + k * 16, KP);
+        wmma::load_matrix_sync(fa, Xrows + k * 16, S::X);
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
-            wmma::load_matrix_sync(fb, W1b + n * 16 * KP + k * 16, KP);  // B(k, n) = W1[n][k]
+            wmma::load_matrix_sync(fb, W1b + n * 16 * S::X + k * 16, S::X);  // B(k, n) = W1[n][k]
             wmma::mma_sync(acc[n], fa, fb, acc[n]);
         }
     }
 #pragma unroll
-    for (int n = 0; n < 2; ++n) wmma::store_matrix_sync(z + n * 16, acc[n], 32, wmma::mem_row_major);
+    for (int n = 0; n < 2; ++n) wmma::store_matrix_sync(z + n * 16, acc[n], S::Z, wmma::mem_row_major);
     __syncwarp();
-    for (int i = lane; i < 16 * 32; i += 32) a1b[i] = __float2bfloat16(fmaxf(z[i] + P[L.b1 + (i & 31)], 0.0f));
+#pragma unroll
+    for (int r = 0; r < 16; ++r) a1b[r * S::B + lane] = __float2bfloat16(fmaxf(z[r * S::Z + lane] + b1, 0.0f));
     __syncwarp();
 #pragma unroll
     for (int n = 0; n < 2; ++n) wmma::fill_fragment(acc[n], 0.0f);
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-        wmma::load_matrix_sync(fa, a1b + k * 16, 32);
+        wmma::load_matrix_sync(fa, a1b + k * 16, S::B);
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
-            wmma::load_matrix_sync(fb, W2b + n * 16 * 32 + k * 16, 32);
+            wmma::load_matrix_sync(fb, W2b + n * 16 * S::B + k * 16, S::B);
             wmma::mma_sync(acc[n], fa, fb, acc[n]);
         }
     }
 #pragma unroll
-    for (int n = 0; n < 2; ++n) wmma::store_matrix_sync(z + n * 16, acc[n], 32, wmma::mem_row_major);
+    for (int n = 0; n < 2; ++n) wmma::store_matrix_sync(z + n * 16, acc[n], S::Z, wmma::mem_row_major);
     __syncwarp();
-    for (int i = lane; i < 16 * 32; i += 32) z[i] += P[L.b2 + (i & 31)];
+#pragma unroll
+    for (int r = 0; r < 16; ++r) z[r * S::Z + lane] += b2;
     __syncwarp();
     if (lane < 16) {
-        float s = P[L.b3];
-        for (int j = 0; j < 32; ++j) s += fmaxf(z[lane * 32 + j], 0.0f) * P[L.w3 + j];
+        float s = b3;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) s += fmaxf(z[lane * S::Z + j], 0.0f) * sw3[j];
         y16[lane] = s;
     }
     __syncwarp();
@@ -415,16 +440,19 @@ __device__ __forceinline__ float mlp_warp_forward_rows(const __nv_bfloat16* X, c
     return lo + P32[3 * MLP_H];
 }
 
-// Shared-memory carve-up of the MLP kernels (bytes): the BF16 weights once
-// per block, then per warp: X tile, A1 (bf16), Z (float), dZ2 and dZ1
-// (bf16), scratch (float), y.
+// Shared-memory carve-up of the MLP kernels (bytes).  Forward: the BF16
+// weights once per block and an X tile per warp.  Backward: the weights and
+// w3 once per block, then per warp X tile, A1 (bf16), Z (float), dZ2 and dZ1
+// (bf16), scratch (float), y, in the strides of MlpPad.
 template <int KP>
 struct MlpSmem {
+    using P = MlpPad<KP>;
     static constexpr int W1 = MLP_H * KP * 2, W2 = MLP_H * MLP_H * 2;
     static constexpr int XW = 16 * KP * 2;
-    static constexpr int A1 = 16 * 32 * 2, Z = 16 * 32 * 4, G = 16 * 32 * 2, Y = 16 * 4;
-    static constexpr int PER_WARP = XW + A1 + Z + 2 * G + Z + Y;
-    static constexpr int bytes(int warps) { return W1 + W2 + warps * PER_WARP; }
+    static constexpr int BW1 = MLP_H * P::X * 2, BW2 = MLP_H * P::B * 2, BW3 = MLP_H * 4;
+    static constexpr int BX = 16 * P::X * 2, A1 = 16 * P::B * 2, Z = 16 * P::Z * 4, G = 16 * P::B * 2, Y = 16 * 4;
+    static constexpr int PER_WARP = BX + A1 + Z + 2 * G + Z + Y;
+    static constexpr int bytes(int warps) { return BW1 + BW2 + BW3 + warps * PER_WARP; }
     static constexpr int fwd_bytes(int warps) { return W1 + W2 + warps * XW; }
 };
 
@@ -437,20 +465,6 @@ __device__ __forceinline__ void mlp_stage_weights(int KP, const __nv_bfloat16* _
                                                   __nv_bfloat16* sW1, __nv_bfloat16* sW2) {
     for (int i = threadIdx.x; i < MLP_H * KP; i += blockDim.x) sW1[i] = Pb[L.w1 + i];
     for (int i = threadIdx.x; i < MLP_H * MLP_H; i += blockDim.x) sW2[i] = Pb[L.w2 + i];
-}
-
-// Loads 16 rows (rows past M - 1 repeat the last one) into shared memory
-// with 16-byte vectors.
-template <int KP>
-__device__ __forceinline__ void mlp_load_rows(const __nv_bfloat16* __restrict__ X, int M, int r0,
-                                              __nv_bfloat16* sX) {
-    const int lane = threadIdx.x & 31;
-    constexpr int VPR = KP / 8;
-    for (int i = lane; i < 16 * VPR; i += 32) {
-        const int r = min(r0 + i / VPR, M - 1);
-        reinterpret_cast<uint4*>(sX)[i] = reinterpret_cast<const uint4*>(X + (long)r * KP)[i % VPR];
-    }
-    __syncwarp();
 }
 
 // Network output y for M rows.  4 warps per block, grid-stride over 16-row
@@ -517,18 +531,36 @@ __global__ void __launch_bounds__(128) k_mlp_backward(int M, const __nv_bfloat16
     using S = MlpSmem<KP>;
     extern __shared__ __align__(128) unsigned char mlp_smem[];
     __nv_bfloat16* sW1 = reinterpret_cast<__nv_bfloat16*>(mlp_smem);
-    __nv_bfloat16* sW2 = reinterpret_cast<__nv_bfloat16*>(mlp_smem + S::W1);
+    __nv_bfloat16* sW2 = reinterpret_cast<__nv_bfloat16*>(mlp_smem + S::BW1);
+    float* sw3 = reinterpret_cast<float*>(mlp_smem + S::BW1 + S::BW2);
     const int w = threadIdx.x / 32, lane = threadIdx.x % 32;
-    unsigned char* mine = mlp_smem + S::W1 + S::W2 + w * S::PER_WARP;
+    unsigned char* mine = mlp_smem + S::BW1 + S::BW2 + S::BW3 + w * S::PER_WARP;
     __nv_bfloat16* sX = reinterpret_cast<__nv_bfloat16*>(mine);
-    __nv_bfloat16* a1b = reinterpret_cast<__nv_bfloat16*>(mine + S::XW);
-    float* z = reinterpret_cast<float*>(mine + S::XW + S::A1);
-    __nv_bfloat16* g2b = reinterpret_cast<__nv_bfloat16*>(mine + S::XW + S::A1 + S::Z);
-    __nv_bfloat16* g1b = reinterpret_cast<__nv_bfloat16*>(mine + S::XW + S::A1 + S::Z + S::G);
-    float* scr = reinterpret_cast<float*>(mine + S::XW + S::A1 + S::Z + 2 * S::G);
-    float* y16 = reinterpret_cast<float*>(mine + S::XW + S::A1 + S::Z + 2 * S::G + S::Z);
-    mlp_stage_weights(KP, Pb, L, sW1, sW2);
+    __nv_bfloat16* a1b = reinterpret_cast<__nv_bfloat16*>(mine + S::BX);
+    float* z = reinterpret_cast<float*>(mine + S::BX + S::A1);
+    __nv_bfloat16* g2b = reinterpret_cast<__nv_bfloat16*>(mine + S::BX + S::A1 + S::Z);
+    __nv_bfloat16* g1b = reinterpret_cast<__nv_bfloat16*>(mine + S::BX + S::A1 + S::Z + S::G);
+    float* scr = reinterpret_cast<float*>(mine + S::BX + S::A1 + S::Z + 2 * S::G);
+    float* y16 = reinterpret_cast<float*>(mine + S::BX + S::A1 + S::Z + 2 * S::G + S::Z);
+    constexpr int XS = MlpPad<KP>::X, BS = MlpPad<KP>::B, ZS = MlpPad<KP>::Z;
+    for (int i = threadIdx.x; i < MLP_H * KP; i += blockDim.x) sW1[(i / KP) * XS + i % KP] = Pb[L.w1 + i];
+    for (int i = threadIdx.x; i < MLP_H * MLP_H; i += blockDim.x) sW2[(i / MLP_H) * BS + i % MLP_H] = Pb[L.w2 + i];
+    if (threadIdx.x < MLP_H) sw3[threadIdx.x] = P[L.w3 + threadIdx.x];
     __syncthreads();
+    const float b1 = P[L.b1 + lane], b2 = P[L.b2 + lane], b3 = P[L.b3];
+    // the next tile's rows and targets in registers while a tile is processed
+    constexpr int VPR = KP / 8, NV = 16 * VPR / 32;
+    uint4 buf[NV];
+    float tnext = 0.f;
+    auto fetch = [&](int t) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            const int i = lane + 32 * k;
+            const int r = min(t * 16 + i / VPR, M - 1);  // rows past M - 1 repeat the last one
+            buf[k] = reinterpret_cast<const uint4*>(X + (long)r * KP)[i % VPR];
+        }
+        tnext = (lane < 16 && t * 16 + lane < M) ? tgt[t * 16 + lane] : 0.f;
+    };
     const int tiles = (M + 15) / 16;
     const float scale = 2.0f / (float)M;
     wmma::fragment<wmma::accumulator, 16, 16, 16, float> gW2[2][2];
@@ -542,42 +574,51 @@ __global__ void __launch_bounds__(128) k_mlp_backward(int M, const __nv_bfloat16
     }
     float gb1 = 0.f, gb2 = 0.f, gw3 = 0.f, gb3 = 0.f, l2 = 0.f;  // lane j: column j
     const float w3j = P[L.w3 + lane];
+    if ((int)blockIdx.x * 4 + w < tiles) fetch(blockIdx.x * 4 + w);
     for (int t = blockIdx.x * 4 + w; t < tiles; t += gridDim.x * 4) {
         const int r0 = t * 16;
-        mlp_load_rows<KP>(X, M, r0, sX);
-        mlp_warp_forward<KP>(sX, sW1, sW2, P, L, a1b, z, y16);  // z = Z2
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            const int i = lane + 32 * k;
+            *reinterpret_cast<uint4*>(sX + (i / VPR) * XS + (i % VPR) * 8) = buf[k];
+        }
+        const float tcur = tnext;
+        __syncwarp();
+        if (t + (int)gridDim.x * 4 < tiles) fetch(t + gridDim.x * 4);
+        mlp_warp_forward<KP>(sX, sW1, sW2, sw3, b1, b2, b3, a1b, z, y16);  // z = Z2
         float dy = 0.f;
         if (lane < 16 && r0 + lane < M) {
-            const float e = y16[lane] - tgt[r0 + lane];
+            const float e = y16[lane] - tcur;
             dy = scale * e;
             l2 += e * e;
         }
         // dZ2 = dy w3 where Z2 > 0; column sums for b2, w3, b3
+#pragma unroll
         for (int r = 0; r < 16; ++r) {
             const float dyr = __shfl_sync(0xffffffffu, dy, r);
-            const float zz = z[r * 32 + lane];
+            const float zz = z[r * ZS + lane];
             gw3 += dyr * fmaxf(zz, 0.f);
             const float g = (zz > 0.f) ? dyr * w3j : 0.f;
             gb2 += g;
-            g2b[r * 32 + lane] = __float2bfloat16(g);
+            g2b[r * BS + lane] = __float2bfloat16(g);
             gb3 += (lane == 0) ? dyr : 0.f;
         }
         __syncwarp();
-        // gW2 += dZ2^T A1: A(m=j, k=r) = dZ2[r][j] (col-major, ld 32), B(k=r, n=i) = A1[r][i] (row-major)
+        // gW2 += dZ2^T A1: A(m=j, k=r) = dZ2[r][j] (col-major), B(k=r, n=i) = A1[r][i] (row-major)
         {
             wmma::fragment<wmma::matrix_a, 16, 16, 16, __nv_bfloat16, wmma::col_major> fa;
             wmma::fragment<wmma::matrix_b, 16, 16, 16, __nv_bfloat16, wmma::row_major> fb;
 #pragma unroll
             for (int a = 0; a < 2; ++a) {
-                wmma::load_matrix_sync(fa, g2b + a * 16, 32);
+                wmma::load_matrix_sync(fa, g2b + a * 16, BS);
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
-                    wmma::load_matrix_sync(fb, a1b + b * 16, 32);
+                    wmma::load_matrix_sync(fb, a1b + b * 16, BS);
                     wmma::mma_sync(gW2[a][b], fa, fb, gW2[a][b]);
                 }
             }
         }
-        // dA1 = dZ2 W2: A = dZ2 (row-major, ld 32), B(k=j, n=i) = W2[j][i] (row-major, ld 32)
+        // dA1 = dZ2 W2: A = dZ2 (row-major), B(k=j, n=i) = W2[j][i] (row-major)
         {
             wmma::fragment<wmma::matrix_a, 16, 16, 16, __nv_bfloat16, wmma::row_major> fa;
             wmma::fragment<wmma::matrix_b, 16, 16, 16, __nv_bfloat16, wmma::row_major> fb;
@@ -586,34 +627,35 @@ __global__ void __launch_bounds__(128) k_mlp_backward(int M, const __nv_bfloat16
             for (int n = 0; n < 2; ++n) wmma::fill_fragment(acc[n], 0.f);
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
-                wmma::load_matrix_sync(fa, g2b + k * 16, 32);
+                wmma::load_matrix_sync(fa, g2b + k * 16, BS);
 #pragma unroll
                 for (int n = 0; n < 2; ++n) {
-                    wmma::load_matrix_sync(fb, sW2 + k * 16 * 32 + n * 16, 32);
+                    wmma::load_matrix_sync(fb, sW2 + k * 16 * BS + n * 16, BS);
                     wmma::mma_sync(acc[n], fa, fb, acc[n]);
                 }
             }
 #pragma unroll
-            for (int n = 0; n < 2; ++n) wmma::store_matrix_sync(scr + n * 16, acc[n], 32, wmma::mem_row_major);
+            for (int n = 0; n < 2; ++n) wmma::store_matrix_sync(scr + n * 16, acc[n], ZS, wmma::mem_row_major);
         }
         __syncwarp();
         // dZ1 = dA1 where A1 > 0
+#pragma unroll
         for (int r = 0; r < 16; ++r) {
-            const float g = (__bfloat162float(a1b[r * 32 + lane]) > 0.f) ? scr[r * 32 + lane] : 0.f;
+            const float g = (__bfloat162float(a1b[r * BS + lane]) > 0.f) ? scr[r * ZS + lane] : 0.f;
             gb1 += g;
-            g1b[r * 32 + lane] = __float2bfloat16(g);
+            g1b[r * BS + lane] = __float2bfloat16(g);
         }
         __syncwarp();
-        // gW1 += dZ1^T X: A(m=j, k=r) = dZ1[r][j] (col-major, ld 32), B(k=r, n=c) = X[r][c] (row-major, ld KP)
+        // gW1 += dZ1^T X: A(m=j, k=r) = dZ1[r][j] (col-major), B(k=r, n=c) = X[r][c] (row-major)
         {
             wmma::fragment<wmma::matrix_a, 16, 16, 16, __nv_bfloat16, wmma::col_major> fa;
             wmma::fragment<wmma::matrix_b, 16, 16, 16, __nv_bfloat16, wmma::row_major> fb;
 #pragma unroll
             for (int a = 0; a < 2; ++a) {
-                wmma::load_matrix_sync(fa, g1b + a * 16, 32);
+                wmma::load_matrix_sync(fa, g1b + a * 16, BS);
 #pragma unroll
                 for (int b = 0; b < KP / 16; ++b) {
-                    wmma::load_matrix_sync(fb, sX + b * 16, KP);
+                    wmma::load_matrix_sync(fb, sX + b * 16, XS);
                     wmma::mma_sync(gW1[a][b], fa, fb, gW1[a][b]);
                 }
             }
@@ -659,13 +701,44 @@ __global__ void __launch_bounds__(128) k_mlp_backward(int M, const __nv_bfloat16
 // (Kingma & Ba 2015) to the FP32 master weights, refreshing the BF16 copy;
 // c1 = 1 - b1^step, c2 = 1 - b2^step.  Padding columns of W1 and the slots
 // past b3 are not updated (slot b3 + 1 of G is the summed squared error).
-__global__ void k_mlp_adam(MlpLayout L, int nin, int R, const float* __restrict__ partial, float* __restrict__ G,
-                           float* P, __nv_bfloat16* Pb, float* m, float* v, float lr, float b1, float b2, float eps,
-                           float c1, float c2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= L.total) return;
+// A block takes ADAM_COLS columns and stages ADAM_ROWS of their rows at a
+// time with all its threads, so the loads of a stage are in flight together
+// and the additions, in row order, read shared memory (one thread a column
+// walking the rows in global memory waited on 256 of them: 11.5 us at 256
+// rows).
+constexpr int ADAM_COLS = 32, ADAM_ROWS = 128;
+
+__global__ void __launch_bounds__(256) k_mlp_adam(MlpLayout L, int nin, int R, const float* __restrict__ partial,
+                                                  float* __restrict__ G, float* P, __nv_bfloat16* Pb, float* m,
+                                                  float* v, float lr, float b1, float b2, float eps, float c1,
+                                                  float c2) {
+    __shared__ float sP[ADAM_ROWS][ADAM_COLS];
+    const int c0 = blockIdx.x * ADAM_COLS, tid = threadIdx.x;
+    const int col = tid % ADAM_COLS, row = tid / ADAM_COLS;
     float g = 0.f;
-    for (int r = 0; r < R; ++r) g += partial[(long)r * L.total + i];
+    for (int r0 = 0; r0 < R; r0 += ADAM_ROWS) {
+        float x[ADAM_ROWS * ADAM_COLS / 256];
+#pragma unroll
+        for (int k = 0; k < ADAM_ROWS * ADAM_COLS / 256; ++k) {
+            const int r = r0 + row + k * (256 / ADAM_COLS);
+            x[k] = (r < R && c0 + col < L.total) ? partial[(long)r * L.total + c0 + col] : 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < ADAM_ROWS * ADAM_COLS / 256; ++k) sP[row + k * (256 / ADAM_COLS)][col] = x[k];
+        __syncthreads();
+        if (tid < ADAM_COLS) {
+            const int n = min(ADAM_ROWS, R - r0);
+            if (n == ADAM_ROWS) {
+#pragma unroll 32
+                for (int r = 0; r < ADAM_ROWS; ++r) g += sP[r][tid];
+            } else {
+                for (int r = 0; r < n; ++r) g += sP[r][tid];
+            }
+        }
+        __syncthreads();
+    }
+    const int i = c0 + tid;
+    if (tid >= ADAM_COLS || i >= L.total) return;
     G[i] = g;
     const bool pad = (i < L.b1 && (i % L.kp) >= nin) || i > L.b3;
     if (pad) return;

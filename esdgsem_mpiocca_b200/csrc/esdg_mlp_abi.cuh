@@ -122,7 +122,7 @@ int esdg_mlp_adam(int ngl, int rows, const float* partial, float* G, float* P, v
         return mlp_fail("mlp_adam: bad arguments");
     const MlpLayout L = mlp_layout(ngl);
     const float c1 = 1.0f - powf(beta1, (float)step), c2 = 1.0f - powf(beta2, (float)step);
-    k_mlp_adam<<<(L.total + 255) / 256, 256, 0, (cudaStream_t)stream>>>(L, mlp_nin(ngl), rows, partial, G, P,
+    k_mlp_adam<<<(L.total + ADAM_COLS - 1) / ADAM_COLS, 256, 0, (cudaStream_t)stream>>>(L, mlp_nin(ngl), rows, partial, G, P,
                                                                          (__nv_bfloat16*)Pb, m, v, lr, beta1, beta2,
                                                                          eps, c1, c2);
     return mlp_cuda(cudaSuccess, "mlp_adam");
