@@ -47,7 +47,7 @@ def log(*a):
 # element-kernel variants of the engine at N = 4 (index = variant number)
 ELEMENT_KERNELS_N4 = ("k_element_tma<5,2,2>", "k_element_tma<5,3,2>", "k_element_tma<5,2,3>",
                       "k_element_rows<5,30,2,1>", "k_element_rows<5,14,2,2>", "k_element_pair<5,3>",
-                      "k_element_pair<5,4>")
+                      "k_element_pair<5,4>", "k_element_oneshot<5>")
 
 
 def element_kernel_name(dc):

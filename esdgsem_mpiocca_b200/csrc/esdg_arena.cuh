@@ -221,9 +221,8 @@ class Arena : public Engine {
 
     template <int NGL>
     void lambda_range(Range re) {
-        using S = ElemShape<NGL>;
         const long n2 = NGL * NGL;
-        k_lambda<NGL><<<(re.size + S::NE - 1) / S::NE, S::THREADS, 0, stream>>>(
+        k_lambda<NGL><<<lambda_blocks(re.size), 256, 0, stream>>>(
             re.size, q + re.begin * n2 * 3, elem_inst + re.begin, st, phys());
     }
     void ranged_lambda(Range re) {

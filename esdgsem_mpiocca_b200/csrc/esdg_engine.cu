@@ -32,6 +32,7 @@
 #include "esdg_tma.cuh"
 #include "esdg_rows.cuh"
 #include "esdg_pair.cuh"
+#include "esdg_oneshot.cuh"
 #include "esdg_indicator.cuh"
 #include "esdg_analysis.cuh"
 #include "esdg_geometry.cuh"
@@ -192,13 +193,37 @@ class Engine {
         return e == cudaErrorMemoryAllocation ? ESDG_E_NOMEM : ESDG_E_CUDA;
     }
 
+    static constexpr size_t SLAB = (size_t)1 << 18;
+    char* slab = nullptr;
+    size_t slab_used = 0;
+
     template <class T>
     int alloc(T** p, size_t n) {
         if (n == 0) n = 1;
+        // Small arrays (operators, step state, counters) share a slab: a
+        // cudaMalloc and its cudaFree take 0.6 ms, and a solver of a small
+        // mesh was mostly those.
+        const size_t need = (n * sizeof(T) + 255) / 256 * 256;
+        if (need <= SLAB / 16) {
+            if (!slab || slab_used + need > SLAB) {
+                void* v = nullptr;
+                cudaError_t e = cudaMalloc(&v, SLAB);
+                if (e == cudaSuccess) bufs.push_back({v, SLAB});
+                if (e == cudaSuccess) e = cudaMemset(v, 0, SLAB);
+                if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc");
+                slab = static_cast<char*>(v);
+                slab_used = 0;
+            }
+            *p = reinterpret_cast<T*>(slab + slab_used);
+            slab_used += need;
+            bytes += n * sizeof(T);
+            return 0;
+        }
         void* v = nullptr;
-        cudaError_t e = cudaMalloc(&v, n * sizeof(T));
+        // whole 16-byte words: the bulk copy of an odd last tile ends in one
+        cudaError_t e = cudaMalloc(&v, (n * sizeof(T) + 15) / 16 * 16);
         if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc");
-        e = cudaMemset(v, 0, n * sizeof(T));
+        e = cudaMemset(v, 0, (n * sizeof(T) + 15) / 16 * 16);
         if (e != cudaSuccess) return cuda_fail(e, "cudaMemset");
         bufs.push_back({v, n * sizeof(T)});
         bytes += n * sizeof(T);
@@ -216,6 +241,8 @@ class Engine {
         pev.clear();
         for (auto& b : bufs) cudaFree(b.p);
         bufs.clear();
+        slab = nullptr;
+        slab_used = 0;
         bytes = 0;
         if (st_host) { cudaFreeHost(st_host); st_host = nullptr; }
         q = gRK = Qt = Qtmp = nullptr;
@@ -466,7 +493,7 @@ class Engine {
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
             cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop)
             return ResShape{0, 0, 0, 0, 0, 0, 0};
-        return resident_shape(ngl, K, sms, PP || PartialDry);
+        return resident_shape(ngl, K, sms, PP || PartialDry, PartialDry);
     }
 
     int setup_resident() {
@@ -550,11 +577,14 @@ class Engine {
     int face_blocks(long n) {
         const int all = (int)((n + 255) / 256);
         if (!elem_inst) return all;
-        if (n_sms <= 0 && cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
-            n_sms = 148;
-        return std::max(1, std::min(all, n_sms * 4));  // the strided kernels' resident blocks
+        return std::max(1, std::min(all, sm_count() * 4));  // the strided kernels' resident blocks
     }
     int n_sms = 0;
+    int sm_count() {
+        if (n_sms <= 0 && cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+            n_sms = 148;
+        return n_sms;
+    }
 
     template <int NGL, bool STRIDE>
     void launch_face_k(const FaceArgs& a, bool av_grad, int blocks) {
@@ -614,14 +644,13 @@ class Engine {
         return 0;
     }
 
-    // Plain-path element kernel: a persistent bulk-copy-pipelined kernel when
-    // the element count allows 16-byte bulk granularity, else the one-shot
-    // one.  Variants 0..TMA_VARIANTS-1: node-per-thread k_element_tma (CTAs
+    // Plain-path element kernel: persistent, bulk-copy-pipelined.  Variants 0..TMA_VARIANTS-1: node-per-thread k_element_tma (CTAs
     // per SM, pipeline depth); then ROW_VARIANTS line-per-thread
     // k_element_rows (elements per tile).  The autotuner times them on the
     // mesh; esdg_set_element_variant can fix one.
-    static constexpr int ELEM_VARIANTS = TMA_VARIANTS + ROW_VARIANTS + PAIR_VARIANTS;
+    static constexpr int ELEM_VARIANTS = TMA_VARIANTS + ROW_VARIANTS + PAIR_VARIANTS + ONESHOT_VARIANTS;
     static constexpr int PAIR_FIRST = TMA_VARIANTS + ROW_VARIANTS;  // two-nodes-per-thread variants follow
+    static constexpr int ONESHOT = PAIR_FIRST + PAIR_VARIANTS;      // the kernel without a pipeline
     int tma_grid[ELEM_VARIANTS] = {};  // persistent grid sizes (0: not usable)
     int tma_ctas[ELEM_VARIANTS] = {};  // resident CTAs per SM
     int tma_variant = 0;
@@ -721,7 +750,6 @@ class Engine {
         for (auto& c : tma_ctas) c = 0;
         tma_tuned = false;
         tma_variant = 0;
-        if (((long long)K * T::N2) % 2 != 0) return 0;
         int r = setup_tma_variant<NGL, 0>();
         if (!r) r = setup_tma_variant<NGL, 1>();
         if (!r) r = setup_tma_variant<NGL, 2>();
@@ -731,6 +759,13 @@ class Engine {
         }
         if (!r) r = setup_pair_variant<NGL, 0>();
         if (!r) r = setup_pair_variant<NGL, 1>();
+        if (!r) {
+            using S = ElemShape<NGL>;
+            const cudaError_t e =
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&tma_ctas[ONESHOT], k_element_oneshot<NGL>, S::THREADS, 0);
+            if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+            tma_grid[ONESHOT] = (K + S::NE - 1) / S::NE;
+        }
         return r;
     }
 
@@ -768,24 +803,25 @@ class Engine {
         else if (v == TMA_VARIANTS) launch_rows_v<NGL, 0>(ea);
         else if (v == TMA_VARIANTS + 1) launch_rows_v<NGL, 1>(ea);
         else if (v == PAIR_FIRST) launch_pair_v<NGL, 0>(ea);
-        else launch_pair_v<NGL, 1>(ea);
+        else if (v == PAIR_FIRST + 1) launch_pair_v<NGL, 1>(ea);
+        else {
+            using S = ElemShape<NGL>;
+            const int gen = elem_gen(ea);
+            if (gen == 0) launch(k_element_oneshot<NGL, 0>, tma_grid[ONESHOT], S::THREADS, 0, ea);
+            else if (gen == 2) launch(k_element_oneshot<NGL, 2>, tma_grid[ONESHOT], S::THREADS, 0, ea);
+            else launch(k_element_oneshot<NGL, 1>, tma_grid[ONESHOT], S::THREADS, 0, ea);
+        }
     }
 
     template <int NGL>
     void launch_elem_plain(const ElemArgs& ea) {
-        if (tma_grid[tma_variant] > 0) {
-            launch_tma<NGL>(ea, tma_variant);
-        } else {
-            using S = ElemShape<NGL>;
-            launch(k_element<NGL>, (K + S::NE - 1) / S::NE, S::THREADS, 0, ea);
-        }
+        launch_tma<NGL>(ea, tma_variant);
         ++launches;
     }
 
     // Autotuner: times every variant of the element kernel on this mesh in
-    // the step's own update mode, on copies of q and gRK (the state is not
-    // touched), and keeps the fastest; runs once, before the step graph is
-    // captured.  tune_K: elements to cover (the arena's live extent).
+    // the step's own update mode (the state is put back) and keeps the
+    // fastest; runs once, before the step graph is captured.  tune_K: elements to cover (the arena's live extent).
     int tune_K = -1;
 
     template <int NGL>
@@ -800,53 +836,75 @@ class Engine {
         const int Kt = tune_K >= 0 ? tune_K : K;
         if (Kt <= 0) return 0;
         const size_t nd = (size_t)Kt * NGL * NGL * 3;
-        // In a step the element kernel follows kernels that evict its inputs
-        // from L2, so every timed launch here starts after an L2-sized flush;
-        // the variants are interleaved so that none profits from order.
-        const size_t flush_bytes = (size_t)256 << 20;
-        double *tq = nullptr, *tg = nullptr;
-        void* flush = nullptr;
-        if (cudaMalloc(&tq, nd * sizeof(double)) != cudaSuccess || cudaMalloc(&tg, nd * sizeof(double)) != cudaSuccess ||
-            cudaMalloc(&flush, flush_bytes) != cudaSuccess) {
-            cudaFree(tq);
-            cudaFree(tg);
+        // Each timing is of the step's own sequence on its own buffers, face
+        // kernel then element kernel, twice over, so that the caches hold what
+        // they hold in a step (launches of the element kernel alone, flushed
+        // or warm, or on copies, order the variants differently on meshes
+        // about the size of L2: 99x99, N = 6: a variant of 188 us a step
+        // where the best has 174).  q and gRK come back from copies (q's in
+        // the scratch of the right-hand side).  The variants are interleaved
+        // so that none profits from order.
+        char* keep = nullptr;
+        if (cudaMalloc(&keep, nd * sizeof(double) + sizeof(DevState)) != cudaSuccess) {
             cudaGetLastError();
-            tma_tuned = false;  // no room for the copies: keep the default variant
+            tma_tuned = false;  // no room for the copy: keep the default variant
             return 0;
         }
-        cudaMemcpyAsync(tq, q, nd * sizeof(double), cudaMemcpyDeviceToDevice, stream);
-        cudaMemcpyAsync(tg, gRK, nd * sizeof(double), cudaMemcpyDeviceToDevice, stream);
-        constexpr int REPS = 5;
-        cudaEvent_t ev[ELEM_VARIANTS][REPS][2];
+        double* kg = reinterpret_cast<double*>(keep);
+        DevState* ts = reinterpret_cast<DevState*>(keep + nd * sizeof(double));
+        cudaMemcpyAsync(Qt, q, nd * sizeof(double), cudaMemcpyDeviceToDevice, stream);
+        cudaMemcpyAsync(kg, gRK, nd * sizeof(double), cudaMemcpyDeviceToDevice, stream);
+        // a running step state (a single mesh's own may be a finished run's)
+        cudaMemsetAsync(ts, 0, sizeof(DevState), stream);
+        DevState* const own = st;
+        if (I == 1) st = ts;
+        constexpr int REPS = 2;
+        const long long launches0 = launches;
+        cudaEvent_t ev[ELEM_VARIANTS + 1][REPS][2];  // the last: the face kernel alone
         for (auto& a2 : ev)
             for (auto& b2 : a2)
                 for (auto& c2 : b2) cudaEventCreate(&c2);
         const bool have = gStages > 0;
         ElemArgs ea = elem_args(rkSSP ? 1 : 0, have ? gA[0] : 0.0, have ? gB[0] : 1.0, have ? gC[0] : 0.0, 0);
-        ea.q = tq;
-        ea.gRK = tg;
         if (AV) { ea.act = act; ea.alist = alist; ea.acount = act + K; }  // the instance that a viscous stage runs
+        // The line-per-thread kernels are not timed: on no mesh measured were
+        // they within 20 % of the best (N = 3: 2.6 times its step, N = 4:
+        // 1.28, N = 5: 1.5), and timing them is a third of the tuning.
+        auto timed = [&](int v) { return tma_grid[v] > 0 && (v < TMA_VARIANTS || v >= PAIR_FIRST); };
         for (int v = 0; v < ELEM_VARIANTS; ++v)
-            if (tma_grid[v] > 0) launch_tma<NGL>(ea, v);  // first-launch costs
+            if (timed(v)) launch_tma<NGL>(ea, v);  // first-launch costs
+        pdl_on = pdl_pays();  // as the step is launched
         for (int r = 0; r < REPS; ++r)
-            for (int v = 0; v < ELEM_VARIANTS; ++v) {
-                if (tma_grid[v] <= 0) continue;
-                cudaMemsetAsync(flush, r + v, flush_bytes, stream);
+            for (int v = 0; v <= ELEM_VARIANTS; ++v) {
+                if (v < ELEM_VARIANTS && !timed(v)) continue;
                 cudaEventRecord(ev[v][r][0], stream);
-                launch_tma<NGL>(ea, v);
+                chained = false;
+                for (int k = 0; k < 2; ++k) {
+                    launch_face<NGL>(AV != 0);
+                    if (v < ELEM_VARIANTS) launch_tma<NGL>(ea, v);
+                }
                 cudaEventRecord(ev[v][r][1], stream);
             }
+        pdl_on = false;
+        launches = launches0;
+        st = own;
+        cudaMemcpyAsync(q, Qt, nd * sizeof(double), cudaMemcpyDeviceToDevice, stream);
+        cudaMemcpyAsync(gRK, kg, nd * sizeof(double), cudaMemcpyDeviceToDevice, stream);
         cudaError_t e = cudaStreamSynchronize(stream);
-        float best = 1e30f;
-        for (int v = 0; v < ELEM_VARIANTS && e == cudaSuccess; ++v) {
-            if (tma_grid[v] <= 0) continue;
-            float sum = 0.0f;
+        float best = 1e30f, face = 0.0f;
+        for (int v = ELEM_VARIANTS; v >= 0 && e == cudaSuccess; --v) {
+            if (v < ELEM_VARIANTS && !timed(v)) continue;
+            float least = 1e30f;
             for (int r = 0; r < REPS && e == cudaSuccess; ++r) {
                 float ms = 0.0f;
                 e = cudaEventElapsedTime(&ms, ev[v][r][0], ev[v][r][1]);
-                sum += ms;
+                least = std::min(least, ms);
             }
-            tma_tune_ms[v] = sum / REPS;
+            if (v == ELEM_VARIANTS) {
+                face = least / 2;
+                continue;
+            }
+            tma_tune_ms[v] = std::max(least / 2 - face, 1e-4f);
             if (e == cudaSuccess && tma_tune_ms[v] < best) {
                 best = tma_tune_ms[v];
                 tma_variant = v;
@@ -855,9 +913,7 @@ class Engine {
         for (auto& a2 : ev)
             for (auto& b2 : a2)
                 for (auto& c2 : b2) cudaEventDestroy(c2);
-        cudaFree(tq);
-        cudaFree(tg);
-        cudaFree(flush);
+        cudaFree(keep);
         if (e != cudaSuccess) return cuda_fail(e, "autotune");
         return 0;
     }
@@ -907,10 +963,11 @@ class Engine {
         }
     }
 
+    int lambda_blocks(int Kn) { return (int)std::min<long long>(((long long)Kn * ngl * ngl + 255) / 256, sm_count() * 8); }
+
     template <int NGL>
     void launch_lambda() {
-        using S = ElemShape<NGL>;
-        k_lambda<NGL><<<(K + S::NE - 1) / S::NE, S::THREADS, 0, stream>>>(K, q, elem_inst, st, phys());
+        k_lambda<NGL><<<lambda_blocks(K), 256, 0, stream>>>(K, q, elem_inst, st, phys());
         ++launches;
     }
 
@@ -1725,7 +1782,7 @@ int esdg_tuned_config(const esdg_deviceclass* d, int* ctas_per_sm, int* stages, 
     if (ctas_per_sm) *ctas_per_sm = E.tma_grid[v] > 0 ? (node_kernel ? esdg::tma_min_blocks(v) : E.tma_ctas[v]) : 0;
     if (ms_variants3)
         for (int k = 0; k < esdg::TMA_VARIANTS; ++k) ms_variants3[k] = E.tma_tune_ms[k];
-    if (stages) *stages = E.tma_grid[v] > 0 ? (node_kernel ? esdg::tma_stages(v) : 2) : 0;
+    if (stages) *stages = E.tma_grid[v] > 0 ? (node_kernel ? esdg::tma_stages(v) : (v == esdg::Engine::ONESHOT ? 1 : 2)) : 0;
     return E.tma_tuned ? ESDG_OK : ESDG_E_ARG;
 }
 
@@ -2088,10 +2145,9 @@ int esdg_diagnostics(int K, int N, const double* wGL, const double* Jinv, const 
 // memory is owned by their own pool allocator, and serving loops that must
 // not stall on cudaMalloc/cudaFree (both synchronise the device).  They pass
 // their own device buffers for the inputs and the output; the scratch this
-// evaluation needs (packed face/side tables, bathymetry traces, face fluxes,
-// a step state) lives in one file-scope device array of fixed size.  The
-// call reads the count of bad connectivity entries back to the host and
-// synchronises its stream before it returns.
+// evaluation needs lives in one file-scope device array of fixed size.
+// The call synchronises its stream before it returns; bad connectivity
+// entries set a pinned host word, and only then is their count read back.
 // ===========================================================================
 namespace esdg {
 
@@ -2118,74 +2174,195 @@ static NoAllocLayout noalloc_layout(int K, int F, int ngl) {
     return L;
 }
 
-// Packs EdgeData / ElemToEdge / MasterSlave / Orientation into the tables the
-// flux and element kernels read, replacing every out-of-range entry by a safe
-// one and counting it, resets the step state, and gathers the bathymetry
-// traces (okl/GatherEdgeData/CollectEdgeData_Bottom.okl:16-134).
-__global__ void k_noalloc_prepare(int K, int F, int ngl, const int* __restrict__ ED, const int* __restrict__ E2E,
-                                  const int* __restrict__ MS, const int* __restrict__ OR, const double* __restrict__ b,
-                                  int4* ftab, int4* side, double* bL, double* bR, DevState* st, int* err) {
+// The scratch a mesh is measured by is that of packed tables, traces and
+// fluxes (the limit callers size their meshes for); the kernels use the flux
+// part and the error count.
+struct RhsArgs {
+    int K, F;
+    const double *q, *Jinv, *Yxi, *Yeta, *Xxi, *Xeta, *Bx, *By, *b, *D, *nx, *ny, *scal;
+    const int *ED, *E2E, *MS, *OR;
+    double *SP, *Qt;   // face-major fluxes [F][3][ngl]; the result
+    int* err;          // count of bad connectivity entries
+    volatile int* flag;  // host word, set where there is one
+    PhysConst c;
+};
+
+__device__ __forceinline__ void rhs_bad(const RhsArgs& a) {
+    atomicAdd(a.err, 1);
+    *a.flag = 1;
+}
+
+// One thread per face node: connectivity checked and read where it is used
+// (an out-of-range entry is replaced by a safe one and counted), both traces
+// and bathymetry traces (okl/GatherEdgeData/CollectEdgeData_Bottom.okl:16-134)
+// straight from q and b, the ES flux.  Two launches and no copy where a call
+// took a memset, a table kernel, two kernels and a read-back: on a small mesh
+// the call is its launches (24x24, N = 4: 45 us).
+template <int NGL, int NUMFLUX>
+__global__ void __launch_bounds__(256) k_rhs_face(const RhsArgs a) {
+    constexpr int N2 = NGL * NGL;
+    pdl_release();
     const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid == 0) {
-        DevState z;
-        memset(&z, 0, sizeof z);
-        z.T = 1.0;
-        *st = z;
+    if (gid >= (long)a.F * NGL) return;
+    const int f = (int)(gid / NGL), i = (int)(gid % NGL);
+    const int* r = a.ED + (long)f * 8;
+    int eL = r[0], eR = r[1], sL = r[2], sR = r[3];
+    const int same = r[4] ? 1 : 0, cpuL = r[5], cpuR = r[6];
+    const double nx = a.nx[gid], ny = a.ny[gid], sc = a.scal[gid];
+    bool bad = false;
+    if (eL < 0 || eL >= a.K || sL < 0 || sL > 3 || cpuL != 0) { bad = true; eL = 0; sL = 0; }
+    if (cpuR == -1) eR = -1;
+    else if (cpuR != 0 || eR < 0 || eR >= a.K || sR < 0 || sR > 3) { bad = true; eR = -1; }
+    if (bad && i == 0) rhs_bad(a);
+    const int ir = same ? i : NGL - 1 - i;
+    const double* qe = a.q + (long)eL * 3 * N2;
+    const int oL = trace_offset(sL, i, NGL);
+    const double hL = qe[oL], huL = qe[oL + N2], hvL = qe[oL + 2 * N2], bLx = a.b[(long)eL * N2 + oL];
+    double hR, huR, hvR, bRx;
+    if (eR >= 0) {
+        const double* qr = a.q + (long)eR * 3 * N2;
+        const int o = trace_offset(sR, ir, NGL);
+        hR = qr[o]; huR = qr[o + N2]; hvR = qr[o + 2 * N2];
+        bRx = a.b[(long)eR * N2 + o];
+    } else {
+        const long exr = (long)f * NGL + ir;
+        const int o = trace_offset(sL, ir, NGL);
+        wall_ghost(a.nx[exr], a.ny[exr], qe[o], qe[o + N2], qe[o + 2 * N2], hR, huR, hvR);
+        bRx = a.b[(long)eL * N2 + o];
     }
-    if (gid < F) {
-        const int* r = ED + gid * 8;
-        int eL = r[0], eR = r[1], sL = r[2], sR = r[3], same = r[4] ? 1 : 0, cpuL = r[5], cpuR = r[6];
-        int bad = 0;
-        if (eL < 0 || eL >= K || sL < 0 || sL > 3 || cpuL != 0) { bad = 1; eL = 0; sL = 0; }
-        if (cpuR == -1) eR = -1;
-        else if (cpuR != 0 || eR < 0 || eR >= K || sR < 0 || sR > 3) { bad = 1; eR = -1; }
-        if (eR < 0) sR = 0;
-        if (bad) atomicAdd(err, 1);
-        ftab[gid] = make_int4(eL, eR, sL | (sR << 2) | (same << 4), 0);
-        const int n2 = ngl * ngl;
-        for (int i = 0; i < ngl; ++i) {
-            const double vl = b[(long)eL * n2 + trace_offset(sL, i, ngl)];
-            bL[gid * ngl + i] = vl;
-            bR[gid * ngl + i] = (eR >= 0) ? b[(long)eR * n2 + trace_offset(sR, i, ngl)] : vl;
+    double F0, F1, F2;
+    es_flux<NUMFLUX>(a.c, nx, ny, hL, huL, hvL, hR, huR, hvR, bLx, bRx, F0, F1, F2);
+    double* sp = a.SP + (long)f * 3 * NGL + i;
+    sp[0] = sc * a.c.geomFace * F0;
+    sp[NGL] = sc * a.c.geomFace * F1;
+    sp[2 * NGL] = sc * a.c.geomFace * F2;
+}
+
+// NE elements per block, one thread per node: the volume term while the face
+// kernel runs (it reads none of its results), then the lift of the element's
+// sides.  Arithmetic as k_element_tma.
+template <int NGL>
+__global__ void __launch_bounds__(ElemShape<NGL>::THREADS) k_rhs_element(const RhsArgs a) {
+    constexpr int N2 = NGL * NGL, NE = ElemShape<NGL>::NE, ND = NE * N2;
+    __shared__ double sD[N2];
+    __shared__ double sh[ND], shu[ND], shv[ND], su[ND], sv[ND], sh2[ND];
+    __shared__ double sYe[ND], sYx[ND], sXe[ND], sXx[ND];
+    const int tid = threadIdx.x;
+    const int el = tid / N2, nd = tid % N2;
+    const int e = blockIdx.x * NE + el;
+    const bool active = e < a.K;
+    const int xi = nd % NGL, eta = nd / NGL;
+    if (tid < N2) sD[tid] = a.D[tid];
+    const long xid = (long)e * N2 + nd, qid = (long)e * 3 * N2 + nd;
+    const int s = el * N2 + nd;
+    double h = 0, hu = 0, hv = 0, J = 0, bx = 0, by = 0;
+    long fo[2] = {-1, -1};
+    double m[2] = {0.0, 0.0};
+    if (active) {
+        h = a.q[qid]; hu = a.q[qid + N2]; hv = a.q[qid + 2 * N2];
+        sYe[s] = a.Yeta[xid]; sYx[s] = a.Yxi[xid]; sXe[s] = a.Xeta[xid]; sXx[s] = a.Xxi[xid];
+        J = a.Jinv[xid]; bx = a.Bx[xid]; by = a.By[xid];
+#pragma unroll
+        for (int pass = 0; pass < 2; ++pass) {
+            int side = -1, j = 0;
+            if (pass == 0) {
+                if (eta == 0) { side = 0; j = xi; }
+                else if (eta == NGL - 1) { side = 2; j = xi; }
+            } else {
+                if (xi == NGL - 1) { side = 1; j = eta; }
+                else if (xi == 0) { side = 3; j = eta; }
+            }
+            if (side >= 0) {
+                const long id = (long)e * 4 + side;
+                int fc = a.E2E[id] - 1, ms = a.MS[id], orr = a.OR[id];
+                bool bad = false;
+                if (fc < 0 || fc >= a.F) { bad = true; fc = 0; }
+                if (ms != 1 && ms != -1) { bad = true; ms = 1; }
+                if (orr != 0 && orr != 1) { bad = true; orr = 1; }
+                if (bad && j == 0) rhs_bad(a);
+                fo[pass] = (long)fc * 3 * NGL + (orr ? j : NGL - 1 - j);
+                m[pass] = -ms;
+            }
         }
+        sh[s] = h; shu[s] = hu; shv[s] = hv;
+        const double ih = (h > 0) ? 1.0 / h : 0.0;
+        su[s] = hu * ih;
+        sv[s] = hv * ih;
+        sh2[s] = h * h;
     }
-    if (gid < 4l * K) {
-        int fc = E2E[gid] - 1, ms = MS[gid], orr = OR[gid];
-        int bad = 0;
-        if (fc < 0 || fc >= F) { bad = 1; fc = 0; }
-        if (ms != 1 && ms != -1) { bad = 1; ms = 1; }
-        if (orr != 0 && orr != 1) { bad = 1; orr = 1; }
-        if (bad) atomicAdd(err, 1);
-        side[gid] = make_int4(fc, ms, orr, 0);
+    __syncthreads();
+    double r0 = 0, r1 = 0, r2 = 0;
+    if (active) {
+        const int rb = el * N2 + eta * NGL, cb = el * N2 + xi;
+        const double g = a.c.g, uL = su[s], vL = sv[s], h2L = sh2[s];
+        const double ye = sYe[s], yx = sYx[s], xe = sXe[s], xx = sXx[s];
+        double d1 = 0.0, d2 = 0.0, d3 = 0.0;
+#pragma unroll
+        for (int l = 0; l < NGL; ++l) {
+            const int p = rb + l;
+            const double dl = sD[xi * NGL + l];
+            double f1, f2, f3;
+            pair_flux_raw<false>(g, h, hu, hv, uL, vL, h2L, ye, xe, sh[p], shu[p], shv[p], su[p], sv[p], sh2[p], sYe[p],
+                                 sXe[p], f1, f2, f3);
+            d1 += dl * f1; d2 += dl * f2; d3 += dl * f3;
+        }
+#pragma unroll
+        for (int l = 0; l < NGL; ++l) {
+            const int p = cb + l * NGL;
+            const double dl = sD[eta * NGL + l];
+            double g1, g2, g3;
+            pair_flux_raw<true>(g, h, hu, hv, uL, vL, h2L, yx, xx, sh[p], shu[p], shv[p], su[p], sv[p], sh2[p], sYx[p],
+                                sXx[p], g1, g2, g3);
+            d1 += dl * g1; d2 += dl * g2; d3 += dl * g3;
+        }
+        d1 *= 0.25;
+        d2 *= 0.125;
+        d3 *= 0.125;
+        r0 = -J * d1;
+        r1 = -J * d2 - a.c.g * h * bx;
+        r2 = -J * d3 - a.c.g * h * by;
+    }
+    pdl_wait();  // the face fluxes
+    if (active) {
+        const double db = 0.0;
+#pragma unroll
+        for (int pass = 0; pass < 2; ++pass) {
+            if (fo[pass] >= 0) {
+                const double* fp = a.SP + fo[pass];
+                const double f0 = m[pass] * fp[0], f1 = m[pass] * fp[NGL], f2 = m[pass] * fp[2 * NGL];
+                r0 += f0 * J;
+                r1 += J * f1 + J * db;
+                r2 += J * f2 + J * db;
+            }
+        }
+        a.Qt[qid] = r0; a.Qt[qid + N2] = r1; a.Qt[qid + 2 * N2] = r2;
     }
 }
 
 template <int NGL>
-static void noalloc_launch(int K, int F, int NumFlux, const PhysConst& c, const double* q, const double* Jinv,
-                           const double* Yxi, const double* Yeta, const double* Xxi, const double* Xeta,
-                           const double* Bx, const double* By, const double* D, const double* nx, const double* ny,
-                           const double* scal, double* base, const NoAllocLayout& L, double* Qt, cudaStream_t s) {
-    DevState* st = reinterpret_cast<DevState*>(base + L.st);
-    FaceArgs fa{F, reinterpret_cast<const int4*>(base + L.ftab), q, nx, ny, scal, base + L.bL, base + L.bR,
-                base + L.SP, nullptr, nullptr, nullptr, st, c};
-    const long nfn = (long)F * NGL;
-    const int fb = (int)((nfn + 255) / 256);
-    // face-major fluxes with the side table (SIDEOUT / SIDEIN off): the
-    // scratch layout of this entry point
-    if (NumFlux == 0) k_face_flux<NGL, 0, false, false, false><<<fb, 256, 0, s>>>(fa);
-    else if (NumFlux == 2) k_face_flux<NGL, 2, false, false, false><<<fb, 256, 0, s>>>(fa);
-    else k_face_flux<NGL, 3, false, false, false><<<fb, 256, 0, s>>>(fa);
-    ElemArgs ea;
-    memset(&ea, 0, sizeof ea);
-    ea.K = K; ea.Jinv = Jinv; ea.Yxi = Yxi; ea.Yeta = Yeta; ea.Xxi = Xxi; ea.Xeta = Xeta; ea.Bx = Bx; ea.By = By;
-    ea.D = D; ea.SP = base + L.SP; ea.side = reinterpret_cast<const int4*>(base + L.side);
-    ea.q = const_cast<double*>(q); ea.Qt = Qt; ea.st = st; ea.mode = 2; ea.c = c;
+static cudaError_t rhs_launch(const RhsArgs& a, int NumFlux, cudaStream_t s) {
+    const int fb = (int)(((long)a.F * NGL + 255) / 256);
+    if (NumFlux == 0) k_rhs_face<NGL, 0><<<fb, 256, 0, s>>>(a);
+    else if (NumFlux == 2) k_rhs_face<NGL, 2><<<fb, 256, 0, s>>>(a);
+    else k_rhs_face<NGL, 3><<<fb, 256, 0, s>>>(a);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
     using S = ElemShape<NGL>;
-    k_element<NGL, false><<<(K + S::NE - 1) / S::NE, S::THREADS, 0, s>>>(ea);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((a.K + S::NE - 1) / S::NE));
+    cfg.blockDim = dim3(S::THREADS);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_rhs_element<NGL>, a);
 }
 
 static std::mutex g_noalloc_mu;
 static double* g_noalloc_ptr[64] = {nullptr};
+static volatile int* g_noalloc_flag[64] = {nullptr};  // pinned host word per device
 
 }  // namespace esdg
 
@@ -2236,6 +2413,7 @@ extern "C" int esdg_compute_rhs_noalloc(int N, int K, int F, int NumFlux, int ES
         }
     }
     double* base = nullptr;
+    volatile int* flag = nullptr;
     {
         // the device address of the scratch array, looked up once per device
         // (with that device current) on the first call
@@ -2247,38 +2425,52 @@ extern "C" int esdg_compute_rhs_noalloc(int N, int K, int F, int NumFlux, int ES
                 g_create_error = std::string("compute_rhs_noalloc: cudaGetSymbolAddress: ") + cudaGetErrorString(e);
                 return ESDG_E_CUDA;
             }
+            void* hp = nullptr;
+            e = cudaHostAlloc(&hp, sizeof(int), cudaHostAllocMapped);
+            if (e != cudaSuccess) {
+                g_create_error = std::string("compute_rhs_noalloc: cudaHostAlloc: ") + cudaGetErrorString(e);
+                return ESDG_E_CUDA;
+            }
+            g_noalloc_flag[dev] = static_cast<volatile int*>(hp);
             g_noalloc_ptr[dev] = static_cast<double*>(p);
         }
         base = g_noalloc_ptr[dev];
+        flag = g_noalloc_flag[dev];
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    int* err = reinterpret_cast<int*>(base + L.err);
-    e = cudaMemsetAsync(err, 0, sizeof(int), s);
-    if (e != cudaSuccess) { g_create_error = std::string("compute_rhs_noalloc: ") + cudaGetErrorString(e); return ESDG_E_CUDA; }
-    const long np = std::max<long>(F, 4l * K);
-    k_noalloc_prepare<<<(int)((np + 255) / 256), 256, 0, s>>>(
-        K, F, ngl, EdgeData, ElemToEdge, ElemEdgeMasterSlave, ElemEdgeOrientation, b,
-        reinterpret_cast<int4*>(base + L.ftab), reinterpret_cast<int4*>(base + L.side), base + L.bL, base + L.bR,
-        reinterpret_cast<DevState*>(base + L.st), err);
+    int* err = reinterpret_cast<int*>(base + L.err);  // 0 between calls
+    *flag = 0;
     PhysConst c;
     c.g = g_const; c.half_g = 0.5 * g_const; c.fourth_g = 0.25 * g_const;
     c.geomFace = 1.0 / (2.0 / (N * (N + 1.0)));
     c.PosPresTOL = PosPresTOL; c.eps0 = 0; c.sigmaMin = 0; c.sigmaMax = 0; c.ZeroTOL = std::pow(10.0, -5); c.sensor_skip = 0.0;
     c.sensor_full = std::numeric_limits<double>::infinity(); c.ES = ES;
+    RhsArgs ra;
+    ra.K = K; ra.F = F; ra.q = q; ra.Jinv = Jinv; ra.Yxi = y_xi; ra.Yeta = y_eta; ra.Xxi = x_xi; ra.Xeta = x_eta;
+    ra.Bx = Bx; ra.By = By; ra.b = b; ra.D = Dmat; ra.nx = nx; ra.ny = ny; ra.scal = scal;
+    ra.ED = EdgeData; ra.E2E = ElemToEdge; ra.MS = ElemEdgeMasterSlave; ra.OR = ElemEdgeOrientation;
+    ra.SP = base + L.SP; ra.Qt = Qt; ra.err = err; ra.c = c;
+    void* dflag = nullptr;
+    e = cudaHostGetDevicePointer(&dflag, const_cast<int*>(flag), 0);
+    if (e != cudaSuccess) { g_create_error = std::string("compute_rhs_noalloc: ") + cudaGetErrorString(e); return ESDG_E_CUDA; }
+    ra.flag = static_cast<volatile int*>(dflag);
     switch (ngl) {
-        case 2: noalloc_launch<2>(K, F, NumFlux, c, q, Jinv, y_xi, y_eta, x_xi, x_eta, Bx, By, Dmat, nx, ny, scal, base, L, Qt, s); break;
-        case 3: noalloc_launch<3>(K, F, NumFlux, c, q, Jinv, y_xi, y_eta, x_xi, x_eta, Bx, By, Dmat, nx, ny, scal, base, L, Qt, s); break;
-        case 4: noalloc_launch<4>(K, F, NumFlux, c, q, Jinv, y_xi, y_eta, x_xi, x_eta, Bx, By, Dmat, nx, ny, scal, base, L, Qt, s); break;
-        case 5: noalloc_launch<5>(K, F, NumFlux, c, q, Jinv, y_xi, y_eta, x_xi, x_eta, Bx, By, Dmat, nx, ny, scal, base, L, Qt, s); break;
-        case 6: noalloc_launch<6>(K, F, NumFlux, c, q, Jinv, y_xi, y_eta, x_xi, x_eta, Bx, By, Dmat, nx, ny, scal, base, L, Qt, s); break;
-        case 7: noalloc_launch<7>(K, F, NumFlux, c, q, Jinv, y_xi, y_eta, x_xi, x_eta, Bx, By, Dmat, nx, ny, scal, base, L, Qt, s); break;
-        default: noalloc_launch<8>(K, F, NumFlux, c, q, Jinv, y_xi, y_eta, x_xi, x_eta, Bx, By, Dmat, nx, ny, scal, base, L, Qt, s); break;
+        case 2: e = rhs_launch<2>(ra, NumFlux, s); break;
+        case 3: e = rhs_launch<3>(ra, NumFlux, s); break;
+        case 4: e = rhs_launch<4>(ra, NumFlux, s); break;
+        case 5: e = rhs_launch<5>(ra, NumFlux, s); break;
+        case 6: e = rhs_launch<6>(ra, NumFlux, s); break;
+        case 7: e = rhs_launch<7>(ra, NumFlux, s); break;
+        default: e = rhs_launch<8>(ra, NumFlux, s); break;
     }
-    e = cudaGetLastError();
     if (e != cudaSuccess) { g_create_error = std::string("compute_rhs_noalloc: launch: ") + cudaGetErrorString(e); return ESDG_E_CUDA; }
+    e = cudaStreamSynchronize(s);
     int nerr = 0;
-    e = cudaMemcpyAsync(&nerr, err, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess && *flag) {
+        e = cudaMemcpyAsync(&nerr, err, sizeof(int), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, sizeof(int), s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    }
     if (e != cudaSuccess) { g_create_error = std::string("compute_rhs_noalloc: ") + cudaGetErrorString(e); return ESDG_E_CUDA; }
     if (nerr) {
         g_create_error = "compute_rhs_noalloc: " + std::to_string(nerr) + " connectivity entries out of range";

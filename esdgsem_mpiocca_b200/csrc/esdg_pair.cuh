@@ -60,6 +60,7 @@ __global__ void __launch_bounds__(PairShape<NGL>::THREADS, MINB) k_element_pair(
             const int t = blockIdx.x + k * gridDim.x;
             if (t < ntiles) tile_issue<NGL, NE>(a, t, stage + k * P::STAGE_DOUBLES, &bar[k]);
         }
+    double lam_all = 0.0;  // single mesh: this thread's wave-speed maximum over its tiles (NaN sticks)
     int it = 0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
         if (t + gridDim.x >= ntiles) pdl_release();  // the CTA's last tile
@@ -202,8 +203,14 @@ __global__ void __launch_bounds__(PairShape<NGL>::THREADS, MINB) k_element_pair(
             }
         }
         if (a.lam) {
-            warp_lambda<P::THREADS>(lam[0], active[0] && !to_list[0], ins[0], a.st);
-            warp_lambda<P::THREADS>(lam[1], active[1] && !to_list[1], ins[1], a.st);
+            if (GEN != 0 && a.elem_inst) {
+                warp_lambda<P::THREADS>(lam[0], active[0] && !to_list[0], ins[0], a.st);
+                warp_lambda<P::THREADS>(lam[1], active[1] && !to_list[1], ins[1], a.st);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+                    if (active[k] && !to_list[k]) lam_all = (isnan(lam[k]) || lam[k] > lam_all) ? lam[k] : lam_all;
+            }
         }
         __syncthreads();  // stage buffer and su, sv, sh2 free again
         if (tid == 0) {
@@ -214,6 +221,9 @@ __global__ void __launch_bounds__(PairShape<NGL>::THREADS, MINB) k_element_pair(
             }
         }
     }
+    // one atomic per warp and launch (one per warp and tile: the last stage's
+    // launch waited on a single key)
+    if (a.lam && !a.elem_inst) warp_lambda<P::THREADS>(lam_all, true, 0, a.st);
 }
 
 }  // namespace esdg

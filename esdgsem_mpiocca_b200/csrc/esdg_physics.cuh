@@ -23,46 +23,6 @@ struct PhysConst {
     int ES;
 };
 
-// Two-point fluxes F#, G# of okl/DG/VolumeKernelFluxDiffV99.okl:17-57 for
-// the pair (L, R), contracted with the averaged metric terms (a, b):
-//   xi  direction: a = Y_eta, b = X_eta, F = a*f - b*g
-//   eta direction: a = Y_xi,  b = X_xi,  G = -a*f + b*g
-__device__ __forceinline__ void two_point_xi(double fourth_g, double half_g, double hL, double huL, double hvL,
-                                             double iL, double hR, double huR, double hvR, double iR, double aL,
-                                             double aR, double bL, double bR, double& F1, double& F2,
-                                             double& F3) {
-    const double h_A = fourth_g * (hL + hR) * (hL + hR);
-    const double h2_A = 0.5 * (hL * hL + hR * hR);
-    const double hu_A = 0.5 * (huL + huR);
-    const double hv_A = 0.5 * (hvL + hvR);
-    const double u_A = 0.5 * (huL * iL + huR * iR);
-    const double v_A = 0.5 * (hvL * iL + hvR * iR);
-    const double a = 0.5 * (aL + aR);
-    const double b = 0.5 * (bL + bR);
-    const double p = h_A - half_g * h2_A;
-    F1 = a * hu_A - b * hv_A;
-    F2 = a * (hu_A * u_A + p) - b * hv_A * u_A;
-    F3 = a * (hu_A * v_A) - b * (hv_A * v_A + p);
-}
-
-__device__ __forceinline__ void two_point_eta(double fourth_g, double half_g, double hL, double huL, double hvL,
-                                              double iL, double hR, double huR, double hvR, double iR, double aL,
-                                              double aR, double bL, double bR, double& G1, double& G2,
-                                              double& G3) {
-    const double h_A = fourth_g * (hL + hR) * (hL + hR);
-    const double h2_A = 0.5 * (hL * hL + hR * hR);
-    const double hu_A = 0.5 * (huL + huR);
-    const double hv_A = 0.5 * (hvL + hvR);
-    const double u_A = 0.5 * (huL * iL + huR * iR);
-    const double v_A = 0.5 * (hvL * iL + hvR * iR);
-    const double a = 0.5 * (aL + aR);
-    const double b = 0.5 * (bL + bR);
-    const double p = h_A - half_g * h2_A;
-    G1 = -a * hu_A + b * hv_A;
-    G2 = -a * (hu_A * u_A + p) + b * hv_A * u_A;
-    G3 = -a * (hu_A * v_A) + b * (hv_A * v_A + p);
-}
-
 // Entropy-stable interface flux at one face node, L = master side state,
 // R = slave side state in the master's node order, n = master's outward unit
 // normal.  NUMFLUX 0: okl/RiemannSolvers/calcESFlux.okl:17-215;

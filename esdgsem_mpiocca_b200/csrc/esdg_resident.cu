@@ -7,18 +7,20 @@
 // two, while the step graph spends that on each of its 12 launches (their
 // start-up, the drained last wave, the first loads of the next).  Here a
 // stage is
-//   export the traces that elements of other CTAs need (global, L2);
-//   the volume term of the first elements, while the neighbours export;
-//   the face fluxes of this CTA's sides into shared memory (a face between
-//   two CTAs is evaluated by both, from the same operands);
-//   lift, update, limiter, and on the last stage the wave-speed maximum.
+//   the volume term of the first elements, while the neighbours' traces
+//   arrive; the face fluxes of this CTA's sides into shared memory (a face
+//   between two CTAs is evaluated by both, from the same operands);
+//   lift, update, limiter, and on the last stage the wave-speed maximum; the
+//   new traces that elements of other CTAs need go out with the update
+//   (global memory, L2).
 // There is no grid barrier: an exported value is one 16-byte word {value,
 // epoch}, written and read as a single 128-bit access, and the reader polls
 // the word itself until the epoch is this stage's.  That is one L2 round
 // trip where a barrier needs a fence, an atomic and the reads after it.
-// The words alternate between two buffers: a CTA writes stage k + 2's over
-// stage k's only after it has read all its neighbours' words of stage
-// k + 1, which they write when they are done with stage k.  The wave-speed
+// The words alternate between two buffers: a CTA writes stage k + 1's over
+// stage k - 1's in its update of stage k, after it has read all its
+// neighbours' words of stage k, which they wrote when they were done with
+// stage k - 1.  The wave-speed
 // maxima go round in the same way, once a step, one word per CTA.  Epochs
 // grow from launch to launch, so no buffer is cleared.
 // Every CTA takes the step's decisions (dt, end of the run) from the same
@@ -33,8 +35,8 @@
 // where those hold all of a CTA's nodes, else 384 (80 registers, 30 to 140
 // bytes spilled): a second pass over the nodes costs more than the spills
 // (51.8 against 59.6 us a step at 148,000 nodes of N = 4).  Where a CTA has
-// threads to spare, whole warps take the exports and face fluxes while the
-// others run the volume term.
+// threads to spare, whole warps take the face fluxes while the others run
+// the volume term and gather the wave-speed words.
 //
 // Measured (B200, us per step, against the step graph): 15-17 against 37-40
 // up to 25,000 nodes (bound by the latency of the exchange and of the FP64
@@ -61,11 +63,11 @@ struct ResLayout {
     __host__ __device__ static constexpr size_t doubles(int ne, int ep) {
         return (size_t)ne * (13 * N2 + 12 * NGL) + 3 * (size_t)ep * N2 + N2;
     }
-    // face records (int4) and export list (4 ne each); limiter: means (4 ne
-    // doubles) and flags (ne)
-    __host__ __device__ static constexpr size_t bytes(int ne, int ep, bool extra) {
-        return 8 * (doubles(ne, ep) + (extra ? 4 * (size_t)ne : 0)) + 16 * 4 * (size_t)ne +
-               4 * (4 * (size_t)ne + (extra ? ne : 0)) + 32;
+    // face records (int4) and export flags (4 ne each); limiter: means (4 ne
+    // doubles) and flags (ne); partial-dry treatment: flags (ne) and b
+    __host__ __device__ static constexpr size_t bytes(int ne, int ep, bool extra, bool dry) {
+        return 8 * (doubles(ne, ep) + (extra ? 4 * (size_t)ne : 0) + (dry ? (size_t)ne * N2 : 0)) +
+               16 * 4 * (size_t)ne + 4 * (4 * (size_t)ne + (extra ? 2 * ne : 0)) + 32;
     }
 };
 
@@ -134,6 +136,12 @@ __device__ __forceinline__ unsigned long long res_warp_max(unsigned long long ke
 template <int NGL, bool EXTRA, int THREADS>
 __global__ void __launch_bounds__(THREADS, 2) k_resident(const ResArgs a) {
     constexpr int N2 = NGL * NGL;
+    // The exported words go out with the update where a thread's registers
+    // have room for it (the small block: 18.9 -> 16.4 us a step at 256
+    // elements of N = 3), else from the finished state at the next stage's
+    // start (the large block spills for it: 5 % slower at 75,000 nodes), and
+    // behind the limiter.
+    constexpr bool EARLY = THREADS == 256 && !EXTRA;
     extern __shared__ __align__(16) double rsm[];
     __shared__ ResCtl ctl;
     __shared__ unsigned long long s_lam, s_key[2];
@@ -158,8 +166,11 @@ __global__ void __launch_bounds__(THREADS, 2) k_resident(const ResArgs a) {
     double* sh2 = sv + EP * N2;
     double* sD = sh2 + EP * N2;
     double* sAvg = sD + N2;                 // [ne][4] (EXTRA)
-    int* sxl = reinterpret_cast<int*>(sAvg + (EXTRA ? 4 * (size_t)a.ne : 0));  // exported sides
-    int* sneg = sxl + 4 * a.ne;             // [ne] element has a negative depth (EXTRA)
+    // exported sides: flags [ne][4] (EARLY), else a list
+    double* sB = sAvg + (EXTRA ? 4 * (size_t)a.ne : 0);  // [ne][N2] b (partial-dry treatment)
+    int* sexp = reinterpret_cast<int*>(sB + (EXTRA && a.dry_on ? (size_t)a.ne * N2 : 0));
+    int* sneg = sexp + 4 * a.ne;             // [ne] element has a negative depth (EXTRA)
+    int* sdry = sneg + a.ne;                 // [ne] element has a node below PosPresTOL (EXTRA)
 
     if (tid == 0) {
         s_nf = 0;
@@ -185,6 +196,10 @@ __global__ void __launch_bounds__(THREADS, 2) k_resident(const ResArgs a) {
         sYx[i] = a.Yxi[k]; sYe[i] = a.Yeta[k]; sXx[i] = a.Xxi[k]; sXe[i] = a.Xeta[k];
     }
     for (int i = tid; i < N2; i += T) sD[i] = a.D[i];
+    if (EXTRA && a.dry_on) {
+        for (int i = tid; i < ne * N2; i += T) sB[i] = a.B[(size_t)e0 * N2 + i];
+        for (int i = tid; i < ne; i += T) sdry[i] = 0;
+    }
     __syncthreads();
     // Faces to evaluate: those whose master side is here, and those whose
     // slave side is here with the master in another CTA (evaluated there
@@ -197,16 +212,17 @@ __global__ void __launch_bounds__(THREADS, 2) k_resident(const ResArgs a) {
         const int other = master ? t.y : t.x;
         const bool local = other >= e0 && other < e0 + ne;
         if (master || !local) sface[atomicAdd(&s_nf, 1)] = make_int4(f, t.x, t.y, (t.z & 31) | (t.w << 8));
-        if (other >= 0 && !local) sxl[atomicAdd(&s_nx, 1)] = i;
+        const bool out = other >= 0 && !local;
+        if (EARLY) sexp[i] = out;
+        else if (out) sexp[atomicAdd(&s_nx, 1)] = i;
     }
     __syncthreads();
-    const int nfaces = s_nf, nexp = s_nx;
+    const int nfaces = s_nf;
     const int npass = (ne + EP - 1) / EP;
     const int el0 = tid / N2, nd = tid % N2;
     const int xi = nd % NGL, eta = nd / NGL;
     const bool worker = el0 < EP;
-    // threads of the exports and face fluxes: the warps from fbase on, the
-    // node warps having theirs to themselves, or all (fbase = 0)
+    // threads of the face fluxes: the warps from fbase on, or all (fbase = 0)
     const int fbase = a.fbase;
     const int ft = tid - fbase, fn = T - fbase;
     const double g = a.c.g;
@@ -249,13 +265,8 @@ __global__ void __launch_bounds__(THREADS, 2) k_resident(const ResArgs a) {
         r0 = -J * d1;
         r1 = -J * d2 - g * h * sBx[m + nd];
         r2 = -J * d3 - g * h * sBy[m + nd];
-        if (EXTRA && a.dry_on) {
-            double mn = 1.0;  // FindDryElements' minimum
-            for (int k = 0; k < N2; ++k) mn = fmin(q[k], mn);
-            if (mn < a.c.PosPresTOL)
-                pd_volume<NGL>(a.c, a.Dc, a.Dup, a.Ddn, q, a.B + (size_t)(e0 + el) * N2, eta, xi, ye, yx, xe, xx, J,
-                               r1, r2);
-        }
+        if (EXTRA && a.dry_on && sdry[el])
+            pd_volume<NGL>(a.c, a.Dc, a.Dup, a.Ddn, q, sB + el * N2, eta, xi, ye, yx, xe, xx, J, r1, r2);
     };
     auto scratch = [&](int el) {
         const double* q = sq + el * 3 * N2;
@@ -264,6 +275,8 @@ __global__ void __launch_bounds__(THREADS, 2) k_resident(const ResArgs a) {
         su[el0 * N2 + nd] = q[nd + N2] * ih;
         sv[el0 * N2 + nd] = q[nd + 2 * N2] * ih;
         sh2[el0 * N2 + nd] = h * h;
+        // FindDryElements: min(1, h) < PosPresTOL (NaN passes by)
+        if (EXTRA && a.dry_on && (h < a.c.PosPresTOL || 1.0 < a.c.PosPresTOL)) sdry[el] = 1;
     };
     double lam = 0.0;   // this thread's wave-speed maximum of the step (NaN sticks)
     auto fold = [&](double v) { lam = (isnan(v) || v > lam) ? v : lam; };
@@ -292,6 +305,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_resident(const ResArgs a) {
             }
         }
         const double h = q[0], hu = q[N2], hv = q[2 * N2];
+        if (EXTRA && a.dry_on && nd == 0) sdry[el] = 0;  // read by this pass's volume terms, behind a barrier
         double q0, q1, q2;
         if (!a.ssp) {
             const double g0 = A * gk[0] + r0, g1 = A * gk[N2] + r1, g2 = A * gk[2 * N2] + r2;
@@ -311,23 +325,44 @@ __global__ void __launch_bounds__(THREADS, 2) k_resident(const ResArgs a) {
         } else if (last) {
             fold(node_lambda(a.c, q0, q1, q2));
         }
+        if (EARLY) {
+            // the next stage's words, as soon as the values are there
+            ResWord* tr = a.tr + ((epoch + 1) & 1) * half;
+#pragma unroll
+            for (int pass = 0; pass < 2; ++pass) {
+                const int sd = pass == 0 ? (eta == 0 ? 0 : (eta == NGL - 1 ? 2 : -1)) : (xi == NGL - 1 ? 1 : (xi == 0 ? 3 : -1));
+                if (sd >= 0 && sexp[el * 4 + sd]) {
+                    ResWord* o = tr + ((size_t)(e0 + el) * 4 + sd) * 3 * NGL + (pass == 0 ? xi : eta);
+                    res_put(o, (unsigned long long)__double_as_longlong(q0), epoch + 1);
+                    res_put(o + NGL, (unsigned long long)__double_as_longlong(q1), epoch + 1);
+                    res_put(o + 2 * NGL, (unsigned long long)__double_as_longlong(q2), epoch + 1);
+                }
+            }
+        }
     };
+    // words of every exported side for stage ep
+    auto export_all = [&](unsigned long long ep) {
+        ResWord* tr = a.tr + (ep & 1) * half;
+        const int n = (EARLY ? 4 * ne : s_nx) * NGL;
+        for (int i = tid; i < n; i += T) {
+            const int j = i % NGL, k = EARLY ? i / NGL : sexp[i / NGL];
+            if (EARLY && !sexp[k]) continue;
+            const double* q = sq + (k / 4) * 3 * N2 + trace_offset(k & 3, j, NGL);
+            ResWord* o = tr + ((size_t)(e0 + k / 4) * 4 + (k & 3)) * 3 * NGL + j;
+            res_put(o, (unsigned long long)__double_as_longlong(q[0]), ep);
+            res_put(o + NGL, (unsigned long long)__double_as_longlong(q[N2]), ep);
+            res_put(o + 2 * NGL, (unsigned long long)__double_as_longlong(q[2 * N2]), ep);
+        }
+    };
+    if (EARLY) export_all(epoch + 1);
 
     bool leave = false;
     while (!leave) {
         for (int s = 0; s < a.stages; ++s) {
             const bool last = s == a.stages - 1;
             ++epoch;
-            ResWord* tr = a.tr + (epoch & 1) * half;
-            // ---- export ----
-            for (int i = ft; i >= 0 && i < nexp * NGL; i += fn) {
-                const int k = sxl[i / NGL], j = i % NGL;
-                const double* q = sq + (k / 4) * 3 * N2 + trace_offset(k & 3, j, NGL);
-                ResWord* o = tr + ((size_t)(e0 + k / 4) * 4 + (k & 3)) * 3 * NGL + j;
-                res_put(o, (unsigned long long)__double_as_longlong(q[0]), epoch);
-                res_put(o + NGL, (unsigned long long)__double_as_longlong(q[N2]), epoch);
-                res_put(o + 2 * NGL, (unsigned long long)__double_as_longlong(q[2 * N2]), epoch);
-            }
+            const ResWord* tr = a.tr + (epoch & 1) * half;
+            if (!EARLY) export_all(epoch);
             if (s == 0 && tid == 0) {
                 if (ran > 0) res_put(lamw + (ran & 1) * gridDim.x + blockIdx.x, s_lam, epoch);
                 s_lam = 0ull;
@@ -386,14 +421,33 @@ __global__ void __launch_bounds__(THREADS, 2) k_resident(const ResArgs a) {
                     o[0] = n ? v0 : -v0; o[NGL] = n ? v1 : -v1; o[2 * NGL] = n ? v2 : -v2;
                 }
             }
-            if (s == 0 && ran > 0 && ft >= 0) {
-                // the wave-speed keys of all CTAs; whole warps (fn is a
-                // multiple of 32)
+            if (s == 0 && ran > 0 && (fbase == 0 || ft < 0)) {
+                // the wave-speed keys of all CTAs, by whole warps that have
+                // no face fluxes to form (or all); a thread's words are
+                // requested together, the late ones again
+                const ResWord* lw = lamw + (ran & 1) * gridDim.x;
+                const int gn = fbase == 0 ? T : fbase;
                 unsigned long long key = 0ull;
-                for (int i = ft; i < (int)gridDim.x; i += fn) {
-                    unsigned long long v = 0ull;
-                    ok = ok && res_poll(lamw + (ran & 1) * gridDim.x + i, epoch, a.wait_limit, v);
-                    key = v > key ? v : key;
+                if constexpr (THREADS == 256) {
+                    for (int i0 = tid; i0 < (int)gridDim.x; i0 += 4 * gn) {
+                        ResWord x[4];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            if (i0 + k * gn < (int)gridDim.x) x[k] = res_get(lw + i0 + k * gn);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            if (i0 + k * gn < (int)gridDim.x) {
+                                unsigned long long v = x[k].v;
+                                if (x[k].epoch != epoch) ok = ok && res_poll(lw + i0 + k * gn, epoch, a.wait_limit, v);
+                                key = v > key ? v : key;
+                            }
+                    }
+                } else {
+                    for (int i = tid; i < (int)gridDim.x; i += gn) {
+                        unsigned long long v = 0ull;
+                        ok = ok && res_poll(lw + i, epoch, a.wait_limit, v);
+                        key = v > key ? v : key;
+                    }
                 }
                 key = res_warp_max(key);
                 if ((tid & 31) == 0) atomicMax(&s_key[ran & 1], key);
@@ -530,7 +584,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_resident(const ResArgs a) {
 }
 
 template <int NGL>
-static ResShape shape_of(int K, int sms, bool extra) {
+static ResShape shape_of(int K, int sms, bool extra, bool dry) {
     constexpr int N2 = NGL * NGL;
     ResShape s{0, 0, 0, 0, 0, 0, 0};
     const int ne = (K + 2 * sms - 1) / (2 * sms);
@@ -539,7 +593,7 @@ static ResShape shape_of(int K, int sms, bool extra) {
     s.block = ne * N2 <= 256 ? 256 : 384;
     const int npass = (ne + s.block / N2 - 1) / (s.block / N2);
     s.ep = (ne + npass - 1) / npass;
-    s.smem = ResLayout<NGL>::bytes(ne, s.ep, extra);
+    s.smem = ResLayout<NGL>::bytes(ne, s.ep, extra, dry);
     if (s.smem > (size_t)112 * 1024) return s;  // two CTAs an SM
     // whole warps for the face nodes (at most four sides an element) where
     // all of them fit beside the nodes; else every thread does both
@@ -564,9 +618,9 @@ static ResShape shape_of(int K, int sms, bool extra) {
         default: break;             \
     }
 
-ResShape resident_shape(int ngl, int K, int sms, bool extra) {
+ResShape resident_shape(int ngl, int K, int sms, bool extra, bool dry) {
     ResShape s{0, 0, 0, 0, 0, 0, 0};
-#define ESDG_F(n) s = shape_of<n>(K, sms, extra)
+#define ESDG_F(n) s = shape_of<n>(K, sms, extra, dry)
     ESDG_RES_DISPATCH(ngl, ESDG_F)
 #undef ESDG_F
     return s;

@@ -39,7 +39,7 @@ struct ResShape {
     int ne, ep, grid, threads, block, fbase;
     size_t smem;
 };
-ResShape resident_shape(int ngl, int K, int sms, bool extra);
+ResShape resident_shape(int ngl, int K, int sms, bool extra, bool dry);
 cudaError_t resident_setup(int ngl, const ResShape& s, bool extra);
 cudaError_t resident_launch(const ResArgs& a, const ResShape& s, bool extra, cudaStream_t stream);
 

@@ -89,8 +89,8 @@ __device__ __forceinline__ void rows_issue_tile(const ElemArgs& a, int t, double
     if (t + 1 == a.skip_tile) return;  // test hook: this tile's copies are never issued
     const int e0 = t * NE;
     const int ne = min(NE, a.K - e0);
-    const unsigned qb = (unsigned)(ne * 3 * S::N2 * sizeof(double));
-    const unsigned nb = (unsigned)(ne * S::N2 * sizeof(double));
+    const unsigned qb = (unsigned)(bulk_even(ne * 3 * S::N2) * sizeof(double));
+    const unsigned nb = (unsigned)(bulk_even(ne * S::N2) * sizeof(double));
     const unsigned fbytes = (unsigned)(ne * 12 * NGL * sizeof(double));
     const double* second = (a.mode == 1) ? a.Qtmp : a.gRK;
     const bool need2 = a.mode != 2;
@@ -190,6 +190,7 @@ __global__ void __launch_bounds__(RowShape<NGL, NE, ST>::THREADS, MINB)
             if (t < ntiles) rows_issue_tile<NGL, NE, ST>(a, t, stage + k * S::STAGE_DOUBLES, &bar[k]);
         }
     const double g = a.c.g;
+    double lam_all = 0.0;  // single mesh: this thread's wave-speed maximum over its tiles (NaN sticks)
     int it = 0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
         if (t + gridDim.x >= ntiles) pdl_release();  // the CTA's last tile
@@ -246,7 +247,8 @@ __global__ void __launch_bounds__(RowShape<NGL, NE, ST>::THREADS, MINB)
         // also the barrier between the two sums; a partly dry element reads
         // its neighbours' old h in the update, so such tiles store directly
         const int idle = __syncthreads_or((inb && !active) || (active && a.dry && a.dry[e]));
-        const bool bulk = (a.mode != 2) && !idle;
+        // (an odd node count, the last tile's at most, is no bulk store's)
+        const bool bulk = (a.mode != 2) && !idle && (min(NE, a.K - e0) * N2) % 2 == 0;
         // ---- eta sums, surface lift and update: column ln of element el ----
         double lam = 0.0;
         if (active) {
@@ -330,7 +332,10 @@ __global__ void __launch_bounds__(RowShape<NGL, NE, ST>::THREADS, MINB)
                 }
             }
         }
-        if (a.lam) warp_lambda<S::THREADS>(lam, active && !to_list, ins, a.st);
+        if (a.lam) {
+            if (a.elem_inst) warp_lambda<S::THREADS>(lam, active && !to_list, ins, a.st);
+            else if (active && !to_list) lam_all = (isnan(lam) || lam > lam_all) ? lam : lam_all;
+        }
         if (bulk) fence_proxy_async_smem();  // shared-memory writes before the bulk store reads them
         __syncthreads();                     // stage buffer and xi sums free again
         if (tid == 0) {
@@ -351,6 +356,9 @@ __global__ void __launch_bounds__(RowShape<NGL, NE, ST>::THREADS, MINB)
         }
     }
     if (tid == 0) bulk_wait_all();
+    // one atomic per warp and launch (one per warp and tile: the last stage's
+    // launch waited on a single key)
+    if (a.lam && !a.elem_inst) warp_lambda<S::THREADS>(lam_all, true, 0, a.st);
 }
 
 }  // namespace esdg

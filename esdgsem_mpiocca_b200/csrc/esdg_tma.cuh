@@ -7,8 +7,8 @@
 // X_eta and the element-side face fluxes: all contiguous in the
 // element-major layout) completing on the stage's mbarrier; while the CTA
 // computes tile k the copies of tile k+1 are in flight.  The arithmetic per
-// node is that of k_element (same operands, same order), only the staging
-// differs: no load of the compute phase leaves the shared memory.
+// node is the reference's, operand for operand; no load of the compute phase
+// leaves the shared memory.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -156,6 +156,8 @@ struct TmaShape : TileLayout<NGL, tma_ne(NGL * NGL)> {
         sizeof(double) * (STAGES * (size_t)L::STAGE_DOUBLES + 3 * L::ND + L::N2) + 16 * STAGES;
 };
 
+__device__ __forceinline__ int bulk_even(int n) { return (n + 1) & ~1; }
+
 // Issues the bulk copies of tile t (NE elements) into stage buffer sb (one
 // thread).
 template <int NGL, int NE>
@@ -164,8 +166,10 @@ __device__ __forceinline__ void tile_issue(const ElemArgs& a, int t, double* sb,
     if (t + 1 == a.skip_tile) return;  // test hook: this tile's copies are never issued
     const int e0 = t * S::NE;
     const int ne = min(S::NE, a.K - e0);
-    const unsigned qb = (unsigned)(ne * 3 * S::N2 * sizeof(double));
-    const unsigned nb = (unsigned)(ne * S::N2 * sizeof(double));
+    // an odd node count (the last tile's at most, NE * N2 is even) is rounded
+    // up to 16 bytes: the buffers and the sections have the word
+    const unsigned qb = (unsigned)(bulk_even(ne * 3 * S::N2) * sizeof(double));
+    const unsigned nb = (unsigned)(bulk_even(ne * S::N2) * sizeof(double));
     const unsigned fb = (unsigned)(ne * 12 * NGL * sizeof(double));
     const double* second = (a.mode == 1) ? a.Qtmp : a.gRK;
     const bool need2 = a.mode != 2;
@@ -190,7 +194,10 @@ __device__ __forceinline__ void tma_issue_tile(const ElemArgs& a, int t, double*
 }
 
 // Persistent flux-differencing volume term + surface lift + RK update
-// (same operations as k_element), tiles double-buffered through TMA.
+// (okl/DG/VolumeKernelFluxDiffV99.okl:60-218, okl/DG/SurfaceKernel.okl:17-142,
+// okl/RungeKutta/rkLS.okl:17-89 + UpdateKernelLS.okl:17-78 in mode 0,
+// okl/RungeKutta/UpdateKernelSSP_V1.okl:17-98 in mode 1), tiles double-buffered
+// through TMA.
 // GEN = 0: the plain single-mesh step (no arena, active set, partial-dry
 // treatment or manufactured source), those branches compiled out; 2: an
 // arena or active set without the partial-dry treatment and manufactured
@@ -220,6 +227,7 @@ __global__ void __launch_bounds__(TmaShape<NGL>::THREADS, MINB) k_element_tma(El
             const int t = blockIdx.x + k * gridDim.x;
             if (t < ntiles) tma_issue_tile<NGL>(a, t, stage + k * S::STAGE_DOUBLES, &bar[k]);
         }
+    double lam_all = 0.0;  // single mesh: this thread's wave-speed maximum over its tiles (NaN sticks)
     int it = 0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
         if (t + gridDim.x >= ntiles) pdl_release();  // the CTA's last tile
@@ -346,7 +354,10 @@ __global__ void __launch_bounds__(TmaShape<NGL>::THREADS, MINB) k_element_tma(El
                 if (a.lam) lam = node_lambda(a.c, q0, q1, q2);
             }
         }
-        if (a.lam) warp_lambda<S::THREADS>(lam, active && !to_list, ins, a.st);
+        if (a.lam) {
+            if (GEN != 0 && a.elem_inst) warp_lambda<S::THREADS>(lam, active && !to_list, ins, a.st);
+            else if (active && !to_list) lam_all = (isnan(lam) || lam > lam_all) ? lam : lam_all;
+        }
         __syncthreads();  // stage buffer and si free again
         if (tid == 0) {
             const int tn = t + ST * gridDim.x;
@@ -356,6 +367,9 @@ __global__ void __launch_bounds__(TmaShape<NGL>::THREADS, MINB) k_element_tma(El
             }
         }
     }
+    // one atomic per warp and launch (one per warp and tile: the last stage's
+    // launch waited on a single key)
+    if (a.lam && !a.elem_inst) warp_lambda<S::THREADS>(lam_all, true, 0, a.st);
 }
 
 }  // namespace esdg

@@ -210,22 +210,23 @@ int esdg_compute_rhs_noalloc(int N, int K, int F, int NumFlux, int ES, double g_
 /* Element-kernel variant chosen by the engine's autotuner (no counterpart
  * in the reference): before the first step graph is captured the engine
  * times each compiled variant of the element kernel on the mesh (in the
- * step's own update mode, on copies of q and gRK, each launch after an
- * L2-sized flush) and keeps the fastest.  Variants 0-2: one thread per node
+ * step's own update mode, behind the face kernel as in a step, whose own
+ * time is taken off; the state is put back) and keeps the fastest; a mesh that runs in the chip-resident time loop is tuned when
+ * its variants are asked for.  Variants 0-2: one thread per node
  * (CTAs per SM the register budget is cut for, 2 or 3; bulk-copy pipeline
  * depth, 2 or 3 tiles); variants 3-4 (N = 2..5): one thread per element row
- * and column, each symmetric two-point flux evaluated once (two tile sizes).
- * *ctas_per_sm and *stages receive the choice (0: the one-shot kernel is
- * used), ms_variants3 [3] (may be NULL) the measured launch times of
+ * and column, each symmetric two-point flux evaluated once (two tile sizes);
+ * variants 5-6: two nodes per thread (register budgets); variant 7: one-shot
+ * blocks without a pipeline.
+ * *ctas_per_sm and *stages receive the choice, ms_variants3 [3] (may be NULL) the measured launch times of
  * variants 0-2 (esdg_element_variants reports all of them).
  * ESDG_E_ARG before the tuning ran. */
 int esdg_tuned_config(const esdg_deviceclass* d, int* ctas_per_sm, int* stages, float* ms_variants3);
 
 /* All element-kernel variants (no counterpart in the reference): *count
- * the number compiled, *chosen the one the steps use (-1: the one-shot
- * kernel), and for the first cap of them ms [cap] the autotuner's launch
+ * the number compiled, *chosen the one the steps use, and for the first cap of them ms [cap] the autotuner's launch
  * times (0: not timed) and ctas_per_sm [cap] the resident CTAs per SM
- * (0: not available for this degree / element count).  Pointers may be
+ * (0: not available for this degree).  Pointers may be
  * NULL.  ESDG_E_ARG before the tuning ran (or a variant was fixed). */
 int esdg_element_variants(const esdg_deviceclass* d, int* chosen, int* count, float* ms, int* ctas_per_sm,
                           int cap);
