@@ -87,6 +87,20 @@ __device__ __forceinline__ void mark_active(int* act, int e, int4 nb) {
     if (nb.w >= 0) act[nb.w] = 1;
 }
 
+// Decision counts of a thread into the four totals: one atomic per warp and
+// count (one per thread was 85,000 on four neighbouring words at a full grid:
+// 30 us of the fused pass whatever the mesh).  Whole warps, blockDim.x a
+// multiple of 32 except for a last partial warp.
+__device__ __forceinline__ void add_counts(unsigned long long* stats, const unsigned (&cnt)[4]) {
+    const int first = threadIdx.x & ~31, lanes = min(32, (int)blockDim.x - first);
+    const unsigned mask = lanes == 32 ? 0xffffffffu : (1u << lanes) - 1u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const unsigned n = __reduce_add_sync(mask, cnt[k]);
+        if ((threadIdx.x & 31) == 0 && n) atomicAdd(&stats[k], (unsigned long long)n);
+    }
+}
+
 template <int NGL>
 struct IndShape {
     static constexpr int N2 = NGL * NGL, NE = ElemShape<NGL>::NE, THREADS = NE * N2;
@@ -490,7 +504,7 @@ __global__ void __launch_bounds__(IndShape<NGL>::THREADS, 3) k_indicator(IndArgs
     if (tid < N2) sV[tid] = a.Vinv[tid];
     pdl_wait();
     if (blockIdx.x == 0 && tid == 0) *a.acount = 0;
-    unsigned long long cnt[4] = {0, 0, 0, 0};
+    unsigned cnt[4] = {0, 0, 0, 0};
     constexpr int PF = 2;  // tiles of loads in flight
     int t = blockIdx.x;
     IndLoad ring[PF];
@@ -572,11 +586,7 @@ __global__ void __launch_bounds__(IndShape<NGL>::THREADS, 3) k_indicator(IndArgs
         }
         __syncthreads();  // shared tiles are rewritten next iteration
     }
-    if (a.stats) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (cnt[k]) atomicAdd(&a.stats[k], cnt[k]);
-    }
+    if (a.stats) add_counts(a.stats, cnt);
 }
 
 // The learned indicator in one pass at n = 4 and n = 5.  The feature pass
@@ -654,7 +664,7 @@ __global__ void __launch_bounds__(FusedShape<NGL>::THREADS, 3) k_indicator_fused
     double* sm = sM + el * ES;
     double* sw = sW + el * ES;
     __nv_bfloat16* xr = sX + el * XS;
-    unsigned long long cnt[4] = {0, 0, 0, 0};
+    unsigned cnt[4] = {0, 0, 0, 0};
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int e = t * NE + el;
         const bool inb = e < a.K;
@@ -812,11 +822,7 @@ __global__ void __launch_bounds__(FusedShape<NGL>::THREADS, 3) k_indicator_fused
         }
         __syncwarp();  // the warp's shared rows are rewritten next tile
     }
-    if (a.stats) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (cnt[k]) atomicAdd(&a.stats[k], cnt[k]);
-    }
+    if (a.stats) add_counts(a.stats, cnt);
 }
 
 }  // namespace esdg
