@@ -26,6 +26,11 @@ __global__ void k_fill_int(int* p, long n, int v) {
     if (i < n) p[i] = v;
 }
 
+__global__ void k_fill_face(int4* p, long n, int4 v) {
+    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) p[i] = v;
+}
+
 class Arena : public Engine {
   public:
     struct Range {
@@ -40,7 +45,11 @@ class Arena : public Engine {
     std::vector<Inst> inst;
     std::vector<Range> free_e, free_f;
     std::vector<DevState> st_h;  // host copy of all step states (pinned not needed: small)
-    double* dAv = nullptr;       // staging for per-instance uploads (host)
+    // tables of an instance being added, in arena numbering: kept from add to
+    // add (fresh vectors of this size are page faults, as long as the copies),
+    // as large as the largest instance
+    std::vector<int4> ft_h, sd_h;
+    std::vector<int> ed_h;
 
     static bool take(std::vector<Range>& fl, int n, Range* out) {
         for (size_t k = 0; k < fl.size(); ++k)
@@ -133,8 +142,11 @@ class Arena : public Engine {
         const int n2 = ngl * ngl;
         const size_t nn = (size_t)K_ * n2, nf = (size_t)F_ * ngl;
         // connectivity in arena numbering, validated
-        std::vector<int4> ft(F_), sd((size_t)K_ * 4);
-        std::vector<int> ed((size_t)F_ * 8);
+        std::vector<int4>&ft = ft_h, &sd = sd_h;
+        std::vector<int>& ed = ed_h;
+        ft.resize(F_);
+        sd.resize((size_t)K_ * 4);
+        ed.resize((size_t)F_ * 8);
         auto bad = [&](const char* m) { give(free_e, re); give(free_f, rf); return fail(ESDG_E_ARG, m); };
         for (int f = 0; f < F_; ++f) {
             const int* r = ED_h + (size_t)f * 8;
@@ -241,8 +253,7 @@ class Arena : public Engine {
         if (id < 0 || id >= max_inst || !inst[id].live) return fail(ESDG_E_ARG, "arena: no such live instance");
         Inst& in = inst[id];
         k_fill_int<<<(in.K + 255) / 256, 256, 0, stream>>>(elem_inst + in.e.begin, in.K, max_inst);
-        std::vector<int4> face0((size_t)in.F, make_int4(K_cap, -1, 0, 0));
-        cudaMemcpyAsync(ftab + in.f.begin, face0.data(), face0.size() * sizeof(int4), cudaMemcpyHostToDevice, stream);
+        k_fill_face<<<(in.F + 255) / 256, 256, 0, stream>>>(ftab + in.f.begin, in.F, make_int4(K_cap, -1, 0, 0));
         st_h[id].done = 1;
         cudaMemcpyAsync(&st[id].done, &st_h[id].done, sizeof(int), cudaMemcpyHostToDevice, stream);
         cudaError_t e = cudaStreamSynchronize(stream);
