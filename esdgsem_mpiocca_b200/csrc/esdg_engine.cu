@@ -835,6 +835,19 @@ class Engine {
         }
         const int Kt = tune_K >= 0 ? tune_K : K;
         if (Kt <= 0) return 0;
+        if (NGL == 7 && I == 1 && !AV) {
+            // N = 6 on a single mesh that stays in L2 (about 190 bytes per
+            // node): the one-shot blocks, untimed -- 174 us a step at 480,000
+            // nodes against 181 to 188, and a first loop without the tuning
+            // (4.5 -> 2.2 ms there).  Beyond L2 the pipelined ones win (1.4
+            // million nodes: 469 against 514).
+            int l2 = 0;
+            if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device) == cudaSuccess &&
+                (long long)Kt * NGL * NGL * 190 <= l2) {
+                tma_variant = ONESHOT;
+                return 0;
+            }
+        }
         const size_t nd = (size_t)Kt * NGL * NGL * 3;
         // Each timing is of the step's own sequence on its own buffers, face
         // kernel then element kernel, twice over, so that the caches hold what
@@ -865,7 +878,10 @@ class Engine {
             for (auto& b2 : a2)
                 for (auto& c2 : b2) cudaEventCreate(&c2);
         const bool have = gStages > 0;
-        ElemArgs ea = elem_args(rkSSP ? 1 : 0, have ? gA[0] : 0.0, have ? gB[0] : 1.0, have ? gC[0] : 0.0, 0);
+        // with the zero dt of that state a single mesh's q keeps its values
+        // throughout (SSP: weights 0 and 1), for a reader on another stream
+        ElemArgs ea = rkSSP ? elem_args(1, 0.0, 1.0, have ? gC[0] : 0.0, 0)
+                            : elem_args(0, have ? gA[0] : 0.0, have ? gB[0] : 1.0, have ? gC[0] : 0.0, 0);
         if (AV) { ea.act = act; ea.alist = alist; ea.acount = act + K; }  // the instance that a viscous stage runs
         // The line-per-thread kernels are not timed: on no mesh measured were
         // they within 20 % of the best (N = 3: 2.6 times its step, N = 4:
@@ -1284,14 +1300,16 @@ class Engine {
         return 0;
     }
 
-    // Runs up to nsteps (nsteps <= 0: until done) graph replays.
+    // Runs up to nsteps (nsteps <= 0: until done) steps of a loop whose state
+    // has just been uploaded from st_host (so the first look at it needs no
+    // read-back); on return st_host holds the state the loop ended in.
     int run_steps(long long nsteps) {
         const int chunk = 16;
         long long done_steps = 0;
-        for (;;) {
-            int r = poll_state();
+        for (bool known = true;; known = false) {
+            int r = known ? 0 : poll_state();
             if (r) return r;
-            if (st_host->done) break;
+            if (st_host->done || st_host->status == ST_TIMEOUT) break;
             const bool resident = use_resident();
             long long todo = resident ? RES_STEPS : chunk;
             if (nsteps > 0) {
@@ -1341,7 +1359,6 @@ class Engine {
         graph_stale = true;
         loop_ready = true;
         if ((r = run_steps(max_steps > 0 ? max_steps : 0))) return r;
-        if ((r = poll_state())) return r;
         if (t_out) *t_out = st_host->t;
         if (steps_out) *steps_out = st_host->steps;
         if (st_host->status == ST_NONFINITE)
@@ -1379,7 +1396,6 @@ class Engine {
             cudaError_t e = cudaMemcpyAsync(st, st_host, sizeof(DevState), cudaMemcpyHostToDevice, stream);
             if (e != cudaSuccess) return cuda_fail(e, "state upload");
             if ((r = run_steps(0))) return r;
-            if ((r = poll_state())) return r;
         }
         if (t_out) *t_out = st_host->t;
         if (steps_out) *steps_out = st_host->steps;
@@ -1397,13 +1413,10 @@ class Engine {
         if ((r = poll_state())) return r;
         st_host->T = T;
         st_host->done = 0;
-        st_host->max_steps = 0;
-        cudaError_t e = cudaMemcpyAsync(st, st_host, sizeof(DevState), cudaMemcpyHostToDevice, stream);
-        if (e != cudaSuccess) return cuda_fail(e, "state upload");
         // Enough replays for nsteps; the step cap makes extra replays no-ops.
         const int target = st_host->steps + nsteps;
         st_host->max_steps = target;
-        e = cudaMemcpyAsync(st, st_host, sizeof(DevState), cudaMemcpyHostToDevice, stream);
+        cudaError_t e = cudaMemcpyAsync(st, st_host, sizeof(DevState), cudaMemcpyHostToDevice, stream);
         if (e != cudaSuccess) return cuda_fail(e, "state upload");
         loop_ready = true;
         for (int k = 0; k < nsteps;) {

@@ -3,8 +3,9 @@
 // One RK stage of the plain path is two launches:
 //   face_flux  : one thread per face node gathers the two traces straight
 //                from q (wall ghost on boundary faces), evaluates the ES
-//                Riemann flux once and writes the scaled flux F*[F][3][ngl];
-//   element    : NE elements per block staged in shared memory; flux-
+//                Riemann flux once and writes it to both elements' sides;
+//   element    : (esdg_tma.cuh, esdg_pair.cuh, esdg_rows.cuh,
+//                esdg_oneshot.cuh, whichever is fastest) flux-
 //                differencing volume integral, lifting of the four face
 //                fluxes, low-storage (or SSP) RK update and, on the last
 //                stage, the element wave-speed maximum for the next dt.

@@ -169,10 +169,10 @@ class DeviceClass:
         self._ok(self._L.esdg_debug_bulk_wait_test(self.h, int(wait_limit_cycles), int(skip_tile)))
 
     def set_indicator(self, mode: int, net=None):
-        """Indicator of the artificial-viscosity path: 0 the modal sensor and
-        the viscous terms everywhere (the reference's path), 1 the modal
-        sensor with the active set, 2 the learned indicator (`net`, an
-        indicator.IndicatorNet) with the active set."""
+        """Indicator of the artificial-viscosity path: 0 and 1 the modal
+        sensor, the viscous terms on the active set (they are exactly zero
+        elsewhere; 1 also keeps decision counts), 2 the learned indicator
+        (`net`, an indicator.IndicatorNet) with the active set."""
         P, n, margin = _indicator_params(net) if mode >= 2 else (None, 0, 0.0)
         self._ok(self._L.esdg_set_indicator(self.h, mode, P, n, margin))
 

@@ -95,8 +95,8 @@ class Ensemble:
         return int(self._L.esdg_ensemble_kernel_launches(self.h))
 
     def set_indicator(self, mode: int, net=None):
-        """0: modal sensor and viscous terms everywhere (the reference's
-        path); 1: modal sensor with the active set; 2: the learned indicator
+        """0, 1: modal sensor, the viscous terms on the active set (exactly
+        zero elsewhere; 1 keeps decision counts); 2: the learned indicator
         (indicator.IndicatorNet) with the active set."""
         from .deviceclass import _indicator_params
         P, n, margin = _indicator_params(net) if mode >= 2 else (None, 0, 0.0)

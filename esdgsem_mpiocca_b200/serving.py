@@ -18,8 +18,8 @@ request fills the GPU, every further concurrent request only slows all of
 them down.
 
 The one-at-a-time baseline serves the same stream first-in first-out with
-one single-mesh solver per request (the plain path: modal sensor and viscous
-terms on every element).
+one single-mesh solver per request (the plain path: modal sensor, viscous
+terms where they are not exactly zero).
 
 Request generator (the serving configuration): seeded tsunami scenarios of
 the ensemble generator with K = nel^2, nel in {32, 64, 96, 128, 192, 256},

@@ -247,13 +247,11 @@ int esdg_state_pointers(esdg_deviceclass* d, const double** q, const double** b,
 /* Troubled-cell indicator of the artificial-viscosity path (no counterpart
  * in the reference; call after esdg_build_device_kernels with
  * ArtificialViscosity=1):
- *   mode 0  the reference's path: the modal sensor
- *           (okl/ShockCapturing/ShockCapturing.okl:17-234) and the viscous
- *           terms on every element (the default);
- *   mode 1  the modal sensor with the active set: the BR1 gradient and the
- *           viscous terms run only on elements with viscosity > 0 and their
- *           face neighbours (everywhere else they are exactly zero), so the
- *           solution is the same as with mode 0;
+ *   mode 0  the modal sensor (okl/ShockCapturing/ShockCapturing.okl:17-234),
+ *           the default: the BR1 gradient and the viscous terms run only on
+ *           elements with viscosity > 0 and their face neighbours
+ *           (everywhere else they are exactly zero);
+ *   mode 1  the same, with decision counts (esdg_indicator_stats);
  *   mode 2  the learned indicator with the active set: the network whose
  *           FP32 parameter block (esdg_mlp_layout(N+1).total floats) is
  *           `params` sets viscosity 0 where it predicts
