@@ -835,16 +835,23 @@ class Engine {
         }
         const int Kt = tune_K >= 0 ? tune_K : K;
         if (Kt <= 0) return 0;
-        if (NGL == 7 && I == 1 && !AV) {
-            // N = 6 on a single mesh that stays in L2 (about 190 bytes per
-            // node): the one-shot blocks, untimed -- 174 us a step at 480,000
-            // nodes against 181 to 188, and a first loop without the tuning
-            // (4.5 -> 2.2 ms there).  Beyond L2 the pipelined ones win (1.4
-            // million nodes: 469 against 514).
+        if (I == 1 && (NGL == 7 || ((long long)K * NGL * NGL) % 2 != 0)) {
+            // By rule, untimed (a first loop without the tuning: 2.2 instead
+            // of 4.5 ms at 99x99, N = 6): N = 6 meshes that stay in L2 (about
+            // 190 bytes per node) take the one-shot blocks (174 us a step at
+            // 480,000 nodes against 181 to 188 for the others); an odd node
+            // count (N = 2, 4, 6) is otherwise given its degree's usual best
+            // (us a step, best and worst of the timed: N = 2, 331,776 nodes:
+            // 83 to 91; N = 4, 409,600: 124 to 141; N = 6, 1.4 million: 469
+            // to 514).
             int l2 = 0;
-            if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device) == cudaSuccess &&
-                (long long)Kt * NGL * NGL * 190 <= l2) {
-                tma_variant = ONESHOT;
+            if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device) != cudaSuccess) l2 = 0;
+            const bool in_l2 = (long long)Kt * NGL * NGL * 190 <= l2;
+            int v = -1;
+            if (NGL == 7) v = in_l2 ? ONESHOT : (K % 2 ? PAIR_FIRST + 1 : -1);
+            else v = NGL == 3 ? 1 : PAIR_FIRST;
+            if (v >= 0 && tma_grid[v] > 0) {
+                tma_variant = v;
                 return 0;
             }
         }
