@@ -861,19 +861,26 @@ class Engine {
         // they hold in a step (launches of the element kernel alone, flushed
         // or warm, or on copies, order the variants differently on meshes
         // about the size of L2: 99x99, N = 6: a variant of 188 us a step
-        // where the best has 174).  q and gRK come back from copies (q's in
-        // the scratch of the right-hand side).  The variants are interleaved
-        // so that none profits from order.
+        // where the best has 174).  q and gRK come back from copies of the
+        // tuner's own, which no timed kernel writes.  The variants are
+        // interleaved so that none profits from order.
         char* keep = nullptr;
-        if (cudaMalloc(&keep, nd * sizeof(double) + sizeof(DevState)) != cudaSuccess) {
+        if (cudaMalloc(&keep, 2 * nd * sizeof(double) + sizeof(DevState)) != cudaSuccess) {
             cudaGetLastError();
-            tma_tuned = false;  // no room for the copy: keep the default variant
+            tma_tuned = false;  // no room for the copies: keep the default variant
             return 0;
         }
-        double* kg = reinterpret_cast<double*>(keep);
-        DevState* ts = reinterpret_cast<DevState*>(keep + nd * sizeof(double));
-        cudaMemcpyAsync(Qt, q, nd * sizeof(double), cudaMemcpyDeviceToDevice, stream);
+        double* kq = reinterpret_cast<double*>(keep);
+        double* kg = kq + nd;
+        DevState* ts = reinterpret_cast<DevState*>(kg + nd);
+        cudaMemcpyAsync(kq, q, nd * sizeof(double), cudaMemcpyDeviceToDevice, stream);
         cudaMemcpyAsync(kg, gRK, nd * sizeof(double), cudaMemcpyDeviceToDevice, stream);
+        // No element is flagged while the kernels are timed: a loop that ended
+        // by T or by a pause leaves its last sensor pass's flags, and every
+        // timed launch would list those elements once more, past the list's
+        // end, and write their right-hand sides.  The next step's sensor pass
+        // sets the flags anew.
+        if (AV) cudaMemsetAsync(act, 0, ((size_t)K + 1) * sizeof(int), stream);
         // a running step state (a single mesh's own may be a finished run's)
         cudaMemsetAsync(ts, 0, sizeof(DevState), stream);
         DevState* const own = st;
@@ -911,7 +918,7 @@ class Engine {
         pdl_on = false;
         launches = launches0;
         st = own;
-        cudaMemcpyAsync(q, Qt, nd * sizeof(double), cudaMemcpyDeviceToDevice, stream);
+        cudaMemcpyAsync(q, kq, nd * sizeof(double), cudaMemcpyDeviceToDevice, stream);
         cudaMemcpyAsync(gRK, kg, nd * sizeof(double), cudaMemcpyDeviceToDevice, stream);
         cudaError_t e = cudaStreamSynchronize(stream);
         float best = 1e30f, face = 0.0f;
