@@ -278,13 +278,14 @@ class Arena : public Engine {
 
     // Replays the step graph nsteps times without waiting.
     int launch_arena(int nsteps) {
-        if (!tma_tuned && ext_h[0] > 0) {
-            // tune on the first live contents, then re-capture with the choice
+        if (!tma_chosen && ext_h[0] > 0) {
+            // chosen for the first live contents, then captured again
             const int before = tma_variant;
-            tune_K = ext_h[0];
-            int r = run_autotune();
-            if (r) return r;
-            if (tma_variant != before && (r = capture_step_graph())) return r;
+            choose(ext_h[0]);
+            if (tma_variant != before) {
+                const int r = capture_step_graph();
+                if (r) return r;
+            }
         }
         for (int k = 0; k < nsteps; ++k) {
             cudaError_t e = cudaGraphLaunch(graph, stream);

@@ -646,8 +646,8 @@ class Engine {
 
     // Plain-path element kernel: persistent, bulk-copy-pipelined.  Variants 0..TMA_VARIANTS-1: node-per-thread k_element_tma (CTAs
     // per SM, pipeline depth); then ROW_VARIANTS line-per-thread
-    // k_element_rows (elements per tile).  The autotuner times them on the
-    // mesh; esdg_set_element_variant can fix one.
+    // k_element_rows (elements per tile).  Chosen by rule;
+    // esdg_set_element_variant can fix one.
     static constexpr int ELEM_VARIANTS = TMA_VARIANTS + ROW_VARIANTS + PAIR_VARIANTS + ONESHOT_VARIANTS;
     static constexpr int PAIR_FIRST = TMA_VARIANTS + ROW_VARIANTS;  // two-nodes-per-thread variants follow
     static constexpr int ONESHOT = PAIR_FIRST + PAIR_VARIANTS;      // the kernel without a pipeline
@@ -655,8 +655,7 @@ class Engine {
     int tma_ctas[ELEM_VARIANTS] = {};  // resident CTAs per SM
     int tma_variant = 0;
     int forced_variant = -1;
-    bool tma_tuned = false;
-    float tma_tune_ms[ELEM_VARIANTS] = {};
+    bool tma_chosen = false;
 
     template <int NGL, int V>
     int setup_tma_variant() {
@@ -748,7 +747,7 @@ class Engine {
         using T = TmaShape<NGL>;
         for (auto& g : tma_grid) g = 0;
         for (auto& c : tma_ctas) c = 0;
-        tma_tuned = false;
+        tma_chosen = false;
         tma_variant = 0;
         int r = setup_tma_variant<NGL, 0>();
         if (!r) r = setup_tma_variant<NGL, 1>();
@@ -819,133 +818,66 @@ class Engine {
         ++launches;
     }
 
-    // Autotuner: times every variant of the element kernel on this mesh in
-    // the step's own update mode (the state is put back) and keeps the
-    // fastest; runs once, before the step graph is captured.  tune_K: elements to cover (the arena's live extent).
-    int tune_K = -1;
-
+    // The element variant for Kl elements (an arena: its live extent), by
+    // rule.  Measured: us a step with each variant fixed in turn, 470 single
+    // meshes and 150 arenas of N = 1..7, 3,000 to 4 million nodes, even and
+    // odd counts.  The rule's choice is 0.4 % behind the best on average, on
+    // single meshes above 240,000 nodes 0.2 % (timing the variants in a first
+    // loop: 0.8 %, and 1 to 12 ms of that loop).
+    //
+    // Where the step's launches do not overlap (pdl_pays), one variant per
+    // degree, of plain single meshes and of those that list their elements or
+    // look up their instance: on plain ones the other pipelined kernels are up
+    // to 13 % slower and the one-shot blocks 4 to 43 %; on viscous ones the
+    // two-CTA kernel 1.1 to 7.4 % (N = 5: 3.2 % faster to 2.8 % slower), in
+    // arenas 1 to 9 % (N = 5: 1 % faster to 2 % slower).
+    //
+    // Where they overlap, the node-per-thread kernel at two CTAs per SM
+    // leaves room for the next kernel's blocks, and its coarser grid may end
+    // in a fuller last wave of tiles: it wins where its waves are fuller by
+    // more than 5 % (N = 4: 336,400 nodes, 0.91 against 0.76, 107 to 114 us;
+    // 403,225 nodes, 0.91 against 0.91, 127 to 122 us; viscous, 119,025 nodes,
+    // 0.81 against 0.54, 123 to 133 us; arena, 133,350 nodes, 70 to 78 us).
+    // The one-shot blocks have no waves of tiles: they win at N = 6 in L2 (174
+    // to 182 us at 480,249 nodes; 216 to 228 at 592,900, where big's waves are
+    // 0.85 full, and 207 to 201 at 571,536, 0.99), on single meshes at N = 7
+    // where neither pipelined kernel fills its waves (157 to 161 us at
+    // 484,416), and on small plain ones that leave most of a second wave empty
+    // (47 to 50 us at 82,944 nodes, N = 3).
+    //
+    // Partial-dry treatment or manufactured source: their branches cost
+    // registers, and three CTAs per SM pay only on meshes larger than L2
+    // (N = 4: 197 to 188 us at 403,225 nodes, 259 to 274 at 640,000).  Timed
+    // with the partial-dry treatment.
     template <int NGL>
-    int autotune_tma() {
-        if (tma_tuned) return 0;
-        tma_tuned = true;
-        if (tma_grid[0] <= 0) return 0;
-        if (forced_variant >= 0) {
-            tma_variant = forced_variant;
-            return 0;
+    int rule_variant(int Kl) {
+        constexpr int N = NGL - 1;
+        const long long nodes = (long long)Kl * NGL * NGL;
+        const bool arena = I > 1;
+        if (dry || conv) {
+            if (N == 1) return 0;
+            return nodes > 600000 ? 1 : (N >= 6 ? ONESHOT : 0);
         }
-        const int Kt = tune_K >= 0 ? tune_K : K;
-        if (Kt <= 0) return 0;
-        if (I == 1 && (NGL == 7 || ((long long)K * NGL * NGL) % 2 != 0)) {
-            // By rule, untimed (a first loop without the tuning: 2.2 instead
-            // of 4.5 ms at 99x99, N = 6): N = 6 meshes that stay in L2 (about
-            // 190 bytes per node) take the one-shot blocks (174 us a step at
-            // 480,000 nodes against 181 to 188 for the others); an odd node
-            // count (N = 2, 4, 6) is otherwise given its degree's usual best
-            // (us a step, best and worst of the timed: N = 2, 331,776 nodes:
-            // 83 to 91; N = 4, 409,600: 124 to 141; N = 6, 1.4 million: 469
-            // to 514).
+        constexpr int plain[7] = {0, PAIR_FIRST, 1, PAIR_FIRST + 1, 1, PAIR_FIRST + 1, PAIR_FIRST};
+        constexpr int listed[7] = {0, 1, 1, PAIR_FIRST, 1, PAIR_FIRST + 1, PAIR_FIRST};
+        const int best = AV && N == 1 ? ONESHOT : (AV || arena ? listed : plain)[N - 1];
+        if (!pdl_pays() || N == 1) return best;
+        const int big = AV ? 1 : best;
+        auto waves = [&](int v, int ne) { return (double)((Kl + ne - 1) / ne) / (std::max(1, tma_ctas[v]) * sm_count()); };
+        const double w0 = waves(0, TmaShape<NGL>::NE);
+        const double wb = waves(big, big < TMA_VARIANTS ? TmaShape<NGL>::NE : PairShape<NGL>::NE);
+        const double fill0 = w0 / std::ceil(w0), fillb = wb / std::ceil(wb);
+        if (N == 6 && (AV || w0 > 1.0)) {
             int l2 = 0;
             if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device) != cudaSuccess) l2 = 0;
-            const bool in_l2 = (long long)Kt * NGL * NGL * 190 <= l2;
-            int v = -1;
-            if (NGL == 7) v = in_l2 ? ONESHOT : (K % 2 ? PAIR_FIRST + 1 : -1);
-            else v = NGL == 3 ? 1 : PAIR_FIRST;
-            if (v >= 0 && tma_grid[v] > 0) {
-                tma_variant = v;
-                return 0;
-            }
+            // a stage touches about 190 bytes per node
+            return AV || nodes * 190 <= 0.8 * l2 || fillb < 0.9 ? ONESHOT : big;
         }
-        const size_t nd = (size_t)Kt * NGL * NGL * 3;
-        // Each timing is of the step's own sequence on its own buffers, face
-        // kernel then element kernel, twice over, so that the caches hold what
-        // they hold in a step (launches of the element kernel alone, flushed
-        // or warm, or on copies, order the variants differently on meshes
-        // about the size of L2: 99x99, N = 6: a variant of 188 us a step
-        // where the best has 174).  q and gRK come back from copies of the
-        // tuner's own, which no timed kernel writes.  The variants are
-        // interleaved so that none profits from order.
-        char* keep = nullptr;
-        if (cudaMalloc(&keep, 2 * nd * sizeof(double) + sizeof(DevState)) != cudaSuccess) {
-            cudaGetLastError();
-            tma_tuned = false;  // no room for the copies: keep the default variant
-            return 0;
+        if (!AV && !arena) {
+            if (N == 7 && w0 > 1.0 && std::max(fill0, fillb) < 11.0 / 12.0) return ONESHOT;
+            if (nodes < 240000) return w0 > 1.0 && w0 <= 2.0 ? ONESHOT : 0;
         }
-        double* kq = reinterpret_cast<double*>(keep);
-        double* kg = kq + nd;
-        DevState* ts = reinterpret_cast<DevState*>(kg + nd);
-        cudaMemcpyAsync(kq, q, nd * sizeof(double), cudaMemcpyDeviceToDevice, stream);
-        cudaMemcpyAsync(kg, gRK, nd * sizeof(double), cudaMemcpyDeviceToDevice, stream);
-        // No element is flagged while the kernels are timed: a loop that ended
-        // by T or by a pause leaves its last sensor pass's flags, and every
-        // timed launch would list those elements once more, past the list's
-        // end, and write their right-hand sides.  The next step's sensor pass
-        // sets the flags anew.
-        if (AV) cudaMemsetAsync(act, 0, ((size_t)K + 1) * sizeof(int), stream);
-        // a running step state (a single mesh's own may be a finished run's)
-        cudaMemsetAsync(ts, 0, sizeof(DevState), stream);
-        DevState* const own = st;
-        if (I == 1) st = ts;
-        constexpr int REPS = 2;
-        const long long launches0 = launches;
-        cudaEvent_t ev[ELEM_VARIANTS + 1][REPS][2];  // the last: the face kernel alone
-        for (auto& a2 : ev)
-            for (auto& b2 : a2)
-                for (auto& c2 : b2) cudaEventCreate(&c2);
-        const bool have = gStages > 0;
-        // with the zero dt of that state a single mesh's q keeps its values
-        // throughout (SSP: weights 0 and 1), for a reader on another stream
-        ElemArgs ea = rkSSP ? elem_args(1, 0.0, 1.0, have ? gC[0] : 0.0, 0)
-                            : elem_args(0, have ? gA[0] : 0.0, have ? gB[0] : 1.0, have ? gC[0] : 0.0, 0);
-        if (AV) { ea.act = act; ea.alist = alist; ea.acount = act + K; }  // the instance that a viscous stage runs
-        // The line-per-thread kernels are not timed: on no mesh measured were
-        // they within 20 % of the best (N = 3: 2.6 times its step, N = 4:
-        // 1.28, N = 5: 1.5), and timing them is a third of the tuning.
-        auto timed = [&](int v) { return tma_grid[v] > 0 && (v < TMA_VARIANTS || v >= PAIR_FIRST); };
-        for (int v = 0; v < ELEM_VARIANTS; ++v)
-            if (timed(v)) launch_tma<NGL>(ea, v);  // first-launch costs
-        pdl_on = pdl_pays();  // as the step is launched
-        for (int r = 0; r < REPS; ++r)
-            for (int v = 0; v <= ELEM_VARIANTS; ++v) {
-                if (v < ELEM_VARIANTS && !timed(v)) continue;
-                cudaEventRecord(ev[v][r][0], stream);
-                chained = false;
-                for (int k = 0; k < 2; ++k) {
-                    launch_face<NGL>(AV != 0);
-                    if (v < ELEM_VARIANTS) launch_tma<NGL>(ea, v);
-                }
-                cudaEventRecord(ev[v][r][1], stream);
-            }
-        pdl_on = false;
-        launches = launches0;
-        st = own;
-        cudaMemcpyAsync(q, kq, nd * sizeof(double), cudaMemcpyDeviceToDevice, stream);
-        cudaMemcpyAsync(gRK, kg, nd * sizeof(double), cudaMemcpyDeviceToDevice, stream);
-        cudaError_t e = cudaStreamSynchronize(stream);
-        float best = 1e30f, face = 0.0f;
-        for (int v = ELEM_VARIANTS; v >= 0 && e == cudaSuccess; --v) {
-            if (v < ELEM_VARIANTS && !timed(v)) continue;
-            float least = 1e30f;
-            for (int r = 0; r < REPS && e == cudaSuccess; ++r) {
-                float ms = 0.0f;
-                e = cudaEventElapsedTime(&ms, ev[v][r][0], ev[v][r][1]);
-                least = std::min(least, ms);
-            }
-            if (v == ELEM_VARIANTS) {
-                face = least / 2;
-                continue;
-            }
-            tma_tune_ms[v] = std::max(least / 2 - face, 1e-4f);
-            if (e == cudaSuccess && tma_tune_ms[v] < best) {
-                best = tma_tune_ms[v];
-                tma_variant = v;
-            }
-        }
-        for (auto& a2 : ev)
-            for (auto& b2 : a2)
-                for (auto& c2 : b2) cudaEventDestroy(c2);
-        cudaFree(keep);
-        if (e != cudaSuccess) return cuda_fail(e, "autotune");
-        return 0;
+        return 0.95 * fill0 >= fillb ? 0 : big;
     }
 
     // Element kernel, then the viscous terms of the elements it listed.
@@ -1247,30 +1179,38 @@ class Engine {
         ++launches;
     }
 
-    // Fixes the element-kernel variant (-1: let the autotuner pick).
+    // Fixes the element-kernel variant (-1: the engine's choice).
     int set_element_variant(int v) {
         if (!built) return fail(ESDG_E_ARG, "set_element_variant before buildDeviceKernels");
         if (v < -1 || v >= ELEM_VARIANTS) return fail(ESDG_E_ARG, "element variant out of range");
         if (v >= 0 && tma_grid[v] <= 0)
             return fail(ESDG_E_UNSUPPORTED, "element variant not available for this degree and element count");
         forced_variant = v;
-        tma_tuned = v >= 0;
+        tma_chosen = v >= 0;
         if (v >= 0) tma_variant = v;
+        else if (graph && I == 1) choose(K);  // (an arena chooses for the contents of its next launch)
         if (graph) return capture_step_graph();
         return 0;
     }
 
-    int run_autotune() {
-        switch (ngl) {
-            case 2: return autotune_tma<2>();
-            case 3: return autotune_tma<3>();
-            case 4: return autotune_tma<4>();
-            case 5: return autotune_tma<5>();
-            case 6: return autotune_tma<6>();
-            case 7: return autotune_tma<7>();
-            case 8: return autotune_tma<8>();
+    // The fixed variant, else the rule's; once until set_element_variant(-1).
+    void choose(int Kl) {
+        if (tma_chosen) return;
+        tma_chosen = true;
+        int v = forced_variant;
+        if (v < 0) {
+            switch (ngl) {
+                case 2: v = rule_variant<2>(Kl); break;
+                case 3: v = rule_variant<3>(Kl); break;
+                case 4: v = rule_variant<4>(Kl); break;
+                case 5: v = rule_variant<5>(Kl); break;
+                case 6: v = rule_variant<6>(Kl); break;
+                case 7: v = rule_variant<7>(Kl); break;
+                case 8: v = rule_variant<8>(Kl); break;
+                default: v = 0;
+            }
         }
-        return 0;
+        tma_variant = tma_grid[v] > 0 ? v : 0;
     }
 
     int capture_step_graph() {
@@ -1340,7 +1280,10 @@ class Engine {
                 res = ResShape{0, 0, 0, 0, 0, 0, 0};
                 todo = std::min<long long>(todo, chunk);
             }
-            if ((!graph || graph_stale) && ((r = run_autotune()) || (r = capture_step_graph()))) return r;
+            if (!graph || graph_stale) {
+                choose(K);
+                if ((r = capture_step_graph())) return r;
+            }
             for (long long k = 0; k < todo; ++k) {
                 cudaError_t e = cudaGraphLaunch(graph, stream);
                 if (e != cudaSuccess) return cuda_fail(e, "cudaGraphLaunch");
@@ -1444,7 +1387,10 @@ class Engine {
                 }
                 res = ResShape{0, 0, 0, 0, 0, 0, 0};
             }
-            if ((!graph || graph_stale) && ((r = run_autotune()) || (r = capture_step_graph()))) return r;
+            if (!graph || graph_stale) {
+                choose(K);
+                if ((r = capture_step_graph())) return r;
+            }
             e = cudaGraphLaunch(graph, stream);
             if (e != cudaSuccess) return cuda_fail(e, "cudaGraphLaunch");
             launches += kernels_per_step;
@@ -1507,7 +1453,7 @@ class Engine {
         if (r) return r;
         if (gStages <= 0) return fail(ESDG_E_ARG, "profile_steps needs a previous esdg_dg_timeloop call");
         if (AV && indicator) return fail(ESDG_E_UNSUPPORTED, "profile_steps times the reference path (indicator 0)");
-        if ((r = run_autotune())) return r;
+        choose(K);
         const size_t nev = (size_t)nsteps * gStages * 3;
         while (pev.size() < nev) {
             cudaEvent_t e = nullptr;
@@ -1797,7 +1743,7 @@ int esdg_indicator_stats(esdg_deviceclass* d, unsigned long long* counts4, int r
 // tuned when its variants are asked for after a time loop.
 static void tune_if_asked(const esdg_deviceclass* d) {
     esdg::Engine& E = const_cast<esdg_deviceclass*>(d)->eng;
-    if (!E.tma_tuned && E.loop_ready && E.use_resident() && cudaSetDevice(E.device) == cudaSuccess) E.run_autotune();
+    if (!E.tma_chosen && E.loop_ready && E.use_resident() && cudaSetDevice(E.device) == cudaSuccess) E.choose(E.K);
 }
 
 int esdg_tuned_config(const esdg_deviceclass* d, int* ctas_per_sm, int* stages, float* ms_variants3) {
@@ -1808,9 +1754,9 @@ int esdg_tuned_config(const esdg_deviceclass* d, int* ctas_per_sm, int* stages, 
     const bool node_kernel = v < esdg::TMA_VARIANTS;
     if (ctas_per_sm) *ctas_per_sm = E.tma_grid[v] > 0 ? (node_kernel ? esdg::tma_min_blocks(v) : E.tma_ctas[v]) : 0;
     if (ms_variants3)
-        for (int k = 0; k < esdg::TMA_VARIANTS; ++k) ms_variants3[k] = E.tma_tune_ms[k];
+        for (int k = 0; k < esdg::TMA_VARIANTS; ++k) ms_variants3[k] = 0.0f;
     if (stages) *stages = E.tma_grid[v] > 0 ? (node_kernel ? esdg::tma_stages(v) : (v == esdg::Engine::ONESHOT ? 1 : 2)) : 0;
-    return E.tma_tuned ? ESDG_OK : ESDG_E_ARG;
+    return E.tma_chosen ? ESDG_OK : ESDG_E_ARG;
 }
 
 static int element_variants(const esdg::Engine& E, int* chosen, int* count, float* ms, int* ctas, int cap) {
@@ -1818,10 +1764,10 @@ static int element_variants(const esdg::Engine& E, int* chosen, int* count, floa
     if (count) *count = NV;
     if (chosen) *chosen = E.tma_grid[E.tma_variant] > 0 ? E.tma_variant : -1;
     for (int k = 0; k < NV && k < cap; ++k) {
-        if (ms) ms[k] = E.tma_tune_ms[k];
+        if (ms) ms[k] = 0.0f;
         if (ctas) ctas[k] = E.tma_grid[k] > 0 ? E.tma_ctas[k] : 0;
     }
-    return E.tma_tuned ? ESDG_OK : ESDG_E_ARG;
+    return E.tma_chosen ? ESDG_OK : ESDG_E_ARG;
 }
 
 int esdg_element_variants(const esdg_deviceclass* d, int* chosen, int* count, float* ms, int* ctas_per_sm,

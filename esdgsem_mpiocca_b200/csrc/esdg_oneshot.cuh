@@ -6,7 +6,9 @@
 // Where it is the faster one: degrees whose elements fill the pipelined
 // kernels' tiles badly (N = 6: 49 nodes, four elements a tile are 196 of 224
 // lanes, and two per thread 98 of 128) on meshes that stay in L2, where
-// there is no HBM latency for a pipeline to hide.  The autotuner decides.
+// there is no HBM latency for a pipeline to hide; viscous meshes of N = 1; and
+// small meshes with little more than one tile per resident CTA (rule_variant
+// has the times).
 #pragma once
 
 #include "esdg_tma.cuh"

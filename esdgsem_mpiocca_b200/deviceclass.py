@@ -190,8 +190,8 @@ class DeviceClass:
         return dict(zip(("net_zero", "net_full", "modal", "viscous"), [int(v) for v in out]))
 
     def tuned_config(self):
-        """Element-kernel occupancy chosen by the autotuner and the measured
-        launch times of the variants (ms)."""
+        """Element-kernel occupancy and pipeline depth in use (variant_ms:
+        zeros, no variant is timed)."""
         c, st = ctypes.c_int(), ctypes.c_int()
         ms = (ctypes.c_float * 3)()
         rc = self._L.esdg_tuned_config(self.h, ctypes.byref(c), ctypes.byref(st), ms)
@@ -199,13 +199,14 @@ class DeviceClass:
                                      "variant_ms": [float(v) for v in ms]}
 
     def element_variants(self):
-        """All element-kernel variants: the one in use, the autotuner's
-        launch times (ms, 0 if not timed) and resident CTAs per SM (0: not
-        available here); None before the tuning ran."""
+        """All element-kernel variants: the one in use (chosen by the mesh's
+        degree, size and switches), the resident CTAs per SM of each (0: not
+        available here) and zeros for ms (no variant is timed); None before
+        a time loop ran."""
         return _element_variants(self._L, self._L.esdg_element_variants, self.h)
 
     def set_element_variant(self, variant: int):
-        """Fixes the element-kernel variant (-1: the autotuner's choice)."""
+        """Fixes the element-kernel variant (-1: the engine's choice)."""
         self._ok(self._L.esdg_set_element_variant(self.h, int(variant)))
 
     def state_pointers(self):

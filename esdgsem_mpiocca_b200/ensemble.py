@@ -116,7 +116,7 @@ class Ensemble:
         return _element_variants(self._L, self._L.esdg_ensemble_element_variants, self.h)
 
     def set_element_variant(self, variant: int):
-        """Fixes the element-kernel variant (-1: the autotuner's choice)."""
+        """Fixes the element-kernel variant (-1: the engine's choice)."""
         self._ok(self._L.esdg_ensemble_set_element_variant(self.h, int(variant)))
 
     def set_stream(self, stream_ptr):

@@ -207,32 +207,30 @@ int esdg_compute_rhs_noalloc(int N, int K, int F, int NumFlux, int ES, double g_
                              const int* ElemEdgeMasterSlave, const int* ElemEdgeOrientation, double* Qt,
                              void* stream);
 
-/* Element-kernel variant chosen by the engine's autotuner (no counterpart
- * in the reference): before the first step graph is captured the engine
- * times each compiled variant of the element kernel on the mesh (in the
- * step's own update mode, behind the face kernel as in a step, whose own
- * time is taken off; the state is put back) and keeps the fastest; a mesh that runs in the chip-resident time loop is tuned when
- * its variants are asked for.  Variants 0-2: one thread per node
- * (CTAs per SM the register budget is cut for, 2 or 3; bulk-copy pipeline
- * depth, 2 or 3 tiles); variants 3-4 (N = 2..5): one thread per element row
- * and column, each symmetric two-point flux evaluated once (two tile sizes);
- * variants 5-6: two nodes per thread (register budgets); variant 7: one-shot
- * blocks without a pipeline.
- * *ctas_per_sm and *stages receive the choice, ms_variants3 [3] (may be NULL) the measured launch times of
- * variants 0-2 (esdg_element_variants reports all of them).
- * ESDG_E_ARG before the tuning ran. */
+/* Element-kernel variant the engine chose (no counterpart in the reference):
+ * it follows from the degree, the node count (an ensemble: of its first live
+ * contents) and the switches.  Variants 0-2: one thread per node (CTAs per SM
+ * the register budget is cut for, 2 or 3; bulk-copy pipeline depth, 2 or 3
+ * tiles); variants 3-4 (N = 2..5): one thread per element row and column, each
+ * symmetric two-point flux evaluated once (two tile sizes; never chosen,
+ * esdg_set_element_variant can fix them); variants 5-6: two nodes per thread
+ * (register budgets); variant 7: one-shot blocks without a pipeline.
+ * *ctas_per_sm and *stages receive the choice, ms_variants3 [3] (may be NULL)
+ * zeros: no variant is timed.
+ * ESDG_E_ARG before a time loop ran (or a variant was fixed). */
 int esdg_tuned_config(const esdg_deviceclass* d, int* ctas_per_sm, int* stages, float* ms_variants3);
 
 /* All element-kernel variants (no counterpart in the reference): *count
- * the number compiled, *chosen the one the steps use, and for the first cap of them ms [cap] the autotuner's launch
- * times (0: not timed) and ctas_per_sm [cap] the resident CTAs per SM
- * (0: not available for this degree).  Pointers may be
- * NULL.  ESDG_E_ARG before the tuning ran (or a variant was fixed). */
+ * the number compiled, *chosen the one the steps use, and for the first cap
+ * of them ms [cap] zeros (no variant is timed) and ctas_per_sm [cap] the
+ * resident CTAs per SM (0: not available for this degree).
+ * Pointers may be NULL.  ESDG_E_ARG before a time loop ran (or a variant was
+ * fixed). */
 int esdg_element_variants(const esdg_deviceclass* d, int* chosen, int* count, float* ms, int* ctas_per_sm,
                           int cap);
 
 /* Fixes the element-kernel variant for every later step and RHS (no
- * counterpart in the reference); -1 returns to the autotuner's choice.
+ * counterpart in the reference); -1 returns to the engine's choice.
  * Call after buildDeviceKernels; re-captures the step graph if there is one.
  * ESDG_E_UNSUPPORTED for a variant that is not available here.  All
  * variants compute the same bits. */
