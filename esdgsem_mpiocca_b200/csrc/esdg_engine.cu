@@ -1188,7 +1188,7 @@ class Engine {
         forced_variant = v;
         tma_chosen = v >= 0;
         if (v >= 0) tma_variant = v;
-        else if (graph && I == 1) choose(K);  // (an arena chooses for the contents of its next launch)
+        else if (loop_ready && I == 1) choose(K);  // (an arena chooses for the contents of its next launch)
         if (graph) return capture_step_graph();
         return 0;
     }
@@ -1280,10 +1280,7 @@ class Engine {
                 res = ResShape{0, 0, 0, 0, 0, 0, 0};
                 todo = std::min<long long>(todo, chunk);
             }
-            if (!graph || graph_stale) {
-                choose(K);
-                if ((r = capture_step_graph())) return r;
-            }
+            if ((!graph || graph_stale) && (r = capture_step_graph())) return r;
             for (long long k = 0; k < todo; ++k) {
                 cudaError_t e = cudaGraphLaunch(graph, stream);
                 if (e != cudaSuccess) return cuda_fail(e, "cudaGraphLaunch");
@@ -1315,6 +1312,7 @@ class Engine {
         ESDG_DISPATCH(ngl, launch_lambda);
         graph_stale = true;
         loop_ready = true;
+        choose(K);
         if ((r = run_steps(max_steps > 0 ? max_steps : 0))) return r;
         if (t_out) *t_out = st_host->t;
         if (steps_out) *steps_out = st_host->steps;
@@ -1376,6 +1374,7 @@ class Engine {
         cudaError_t e = cudaMemcpyAsync(st, st_host, sizeof(DevState), cudaMemcpyHostToDevice, stream);
         if (e != cudaSuccess) return cuda_fail(e, "state upload");
         loop_ready = true;
+        choose(K);
         for (int k = 0; k < nsteps;) {
             if (use_resident()) {
                 bool ok = false;
@@ -1387,10 +1386,7 @@ class Engine {
                 }
                 res = ResShape{0, 0, 0, 0, 0, 0, 0};
             }
-            if (!graph || graph_stale) {
-                choose(K);
-                if ((r = capture_step_graph())) return r;
-            }
+            if ((!graph || graph_stale) && (r = capture_step_graph())) return r;
             e = cudaGraphLaunch(graph, stream);
             if (e != cudaSuccess) return cuda_fail(e, "cudaGraphLaunch");
             launches += kernels_per_step;
@@ -1739,16 +1735,8 @@ int esdg_indicator_stats(esdg_deviceclass* d, unsigned long long* counts4, int r
     return d->eng.indicator_stats(counts4, reset);
 }
 
-// The resident loop needs no element kernel, so a mesh that runs in it is
-// tuned when its variants are asked for after a time loop.
-static void tune_if_asked(const esdg_deviceclass* d) {
-    esdg::Engine& E = const_cast<esdg_deviceclass*>(d)->eng;
-    if (!E.tma_chosen && E.loop_ready && E.use_resident() && cudaSetDevice(E.device) == cudaSuccess) E.choose(E.K);
-}
-
 int esdg_tuned_config(const esdg_deviceclass* d, int* ctas_per_sm, int* stages, float* ms_variants3) {
     if (!d) return ESDG_E_ARG;
-    tune_if_asked(d);
     const esdg::Engine& E = d->eng;
     const int v = E.tma_variant;
     const bool node_kernel = v < esdg::TMA_VARIANTS;
@@ -1773,7 +1761,6 @@ static int element_variants(const esdg::Engine& E, int* chosen, int* count, floa
 int esdg_element_variants(const esdg_deviceclass* d, int* chosen, int* count, float* ms, int* ctas_per_sm,
                           int cap) {
     if (!d) return ESDG_E_ARG;
-    tune_if_asked(d);
     return element_variants(d->eng, chosen, count, ms, ctas_per_sm, cap);
 }
 

@@ -47,3 +47,39 @@ def test_variant_by_rule(make, want):
         assert np.isfinite(s.q()).all()
     finally:
         s.close()
+
+
+def test_queries_only_read():
+    """Asked from another thread all through a resident time loop, the variant
+    queries give the choice or nothing, and the loop's result is that of a
+    solver nobody asked."""
+    import threading
+    pr = problems.curved_lake(N=4, nel=20, seed=3, ripple=0.02)
+    out, seen = {}, []
+    for ask in (False, True):
+        s = Solver(pr)
+        stop = threading.Event()
+
+        def watch():
+            while not stop.is_set():
+                seen.append((s.dc.element_variants(), s.dc.tuned_config()))
+
+        t = threading.Thread(target=watch)
+        try:
+            if ask:
+                t.start()
+            first = s.run(T=1e9, max_steps=400)
+            Q = s.rhs()
+            out[ask] = (first, s.dc.advance(400, 1e9), Q, s.q())
+            l0 = s.dc.kernel_launches()
+            final = s.dc.element_variants()
+            assert s.dc.kernel_launches() == l0 <= 8
+        finally:
+            stop.set()
+            if ask:
+                t.join()
+            s.close()
+    assert out[0][:2] == out[1][:2]
+    np.testing.assert_array_equal(out[0][2], out[1][2])
+    np.testing.assert_array_equal(out[0][3], out[1][3])
+    assert seen and all(v is None or v == final for v, _ in seen)
