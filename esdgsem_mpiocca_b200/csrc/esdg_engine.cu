@@ -515,7 +515,8 @@ class Engine {
     }
 
     // Up to nsteps steps (at most RES_STEPS) in one launch.  *ok: false when
-    // the device refused the launch (the caller takes the step graph).
+    // the device cannot hold the cooperative grid (fewer SMs granted than it
+    // has; the caller takes the step graph).
     int launch_resident(int nsteps, bool* ok) {
         ResArgs a;
         std::memset(&a, 0, sizeof a);
@@ -533,11 +534,12 @@ class Engine {
         if (PartialDry) { a.dry_on = dry; a.B = B; a.Dc = DcFD; a.Dup = DupFD; a.Ddn = DdnFD; }
         *ok = true;
         const cudaError_t e = resident_launch(a, res, PP || PartialDry, stream);
-        if (e != cudaSuccess) {
+        if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
             cudaGetLastError();
             *ok = false;
             return 0;
         }
+        if (e != cudaSuccess) return cuda_fail(e, "resident loop");
         ++launches;
         return 0;
     }

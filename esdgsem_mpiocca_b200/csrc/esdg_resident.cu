@@ -583,6 +583,9 @@ __global__ void __launch_bounds__(THREADS, 2) k_resident(const ResArgs a) {
     }
 }
 
+// Dynamic shared memory of a CTA at most: two CTAs an SM.
+constexpr size_t RES_SMEM = (size_t)112 * 1024;
+
 template <int NGL>
 static ResShape shape_of(int K, int sms, bool extra, bool dry) {
     constexpr int N2 = NGL * NGL;
@@ -594,7 +597,7 @@ static ResShape shape_of(int K, int sms, bool extra, bool dry) {
     const int npass = (ne + s.block / N2 - 1) / (s.block / N2);
     s.ep = (ne + npass - 1) / npass;
     s.smem = ResLayout<NGL>::bytes(ne, s.ep, extra, dry);
-    if (s.smem > (size_t)112 * 1024) return s;  // two CTAs an SM
+    if (s.smem > RES_SMEM) return s;
     // whole warps for the face nodes (at most four sides an element) where
     // all of them fit beside the nodes; else every thread does both
     const int nodes = (s.ep * N2 + 31) / 32 * 32, faces = (4 * ne * NGL + 31) / 32 * 32;
@@ -640,8 +643,11 @@ static const void* kernel_of(int ngl, const ResShape& s, bool extra) {
     return k;
 }
 
+// The attribute belongs to the function, not to a solver: always the bound,
+// whatever this mesh needs, or a smaller solver of the same instance would
+// take it from a larger one.
 cudaError_t resident_setup(int ngl, const ResShape& s, bool extra) {
-    return cudaFuncSetAttribute(kernel_of(ngl, s, extra), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+    return cudaFuncSetAttribute(kernel_of(ngl, s, extra), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RES_SMEM);
 }
 
 cudaError_t resident_launch(const ResArgs& a, const ResShape& s, bool extra, cudaStream_t stream) {
