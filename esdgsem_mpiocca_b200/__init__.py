@@ -47,6 +47,7 @@ def _declare(lib):
         "esdg_advance": (_I, [_VP, _I, _D, _PD, _PI]),
         "esdg_profile_steps": (_I, [_VP, _I, _PD, _PD]),
         "esdg_debug_bulk_wait_test": (_I, [_VP, ctypes.c_longlong, _I]),
+        "esdg_debug_resident_wait_test": (_I, [_VP, ctypes.c_longlong]),
         "esdg_set_pause": (_I, [_VP, _D]),
         "esdg_set_indicator_every_stage": (_I, [_VP, _I]),
         "esdg_okada_uplift": (_I, [ctypes.c_longlong, _VP, _VP, _PD, _I, _I, _VP, _VP]),

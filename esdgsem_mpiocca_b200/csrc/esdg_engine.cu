@@ -484,6 +484,16 @@ class Engine {
     double* res_words = nullptr;             // exchanged words: traces, then wave-speed keys
     unsigned long long res_epoch = 0;        // epochs used so far
     static constexpr int RES_STEPS = 1024;   // steps per launch at most
+    // test hook of its bounded waits (esdg_debug_resident_wait_test)
+    long long res_wait_limit = 0;
+
+    int set_resident_wait_test(long long limit) {
+        if (!built) return fail(ESDG_E_ARG, "resident-wait test hook before buildDeviceKernels");
+        if (limit < 0) return fail(ESDG_E_ARG, "resident-wait test hook: limit >= 0");
+        if (res.grid <= 0) return fail(ESDG_E_UNSUPPORTED, "resident-wait test hook: this mesh runs in the step graph");
+        res_wait_limit = limit;
+        return 0;
+    }
 
     // The launch shape, zeros where the step graph has to run: artificial
     // viscosity, analysis outputs, an arena (I > 1), or too many elements.
@@ -532,6 +542,7 @@ class Engine {
         a.stages = gStages; a.ssp = rkSSP; a.numflux = NumFlux; a.nsteps = nsteps;
         a.PP = PP; a.EleSizes = EleSizes; a.GLw = GLw;
         if (PartialDry) { a.dry_on = dry; a.B = B; a.Dc = DcFD; a.Dup = DupFD; a.Ddn = DdnFD; }
+        a.wait_limit = res_wait_limit;
         *ok = true;
         const cudaError_t e = resident_launch(a, res, PP || PartialDry, stream);
         if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
@@ -1256,6 +1267,13 @@ class Engine {
         return 0;
     }
 
+    bool timed_out() const { return st_host->status == ST_TIMEOUT || st_host->status == ST_PEER_TIMEOUT; }
+    int fail_timed_out() {
+        return fail(ESDG_E_CUDA, st_host->status == ST_TIMEOUT
+                                     ? "a bulk copy did not complete (bounded wait)"
+                                     : "a neighbour's trace did not arrive in the chip-resident loop (bounded wait)");
+    }
+
     // Runs up to nsteps (nsteps <= 0: until done) steps of a loop whose state
     // has just been uploaded from st_host (so the first look at it needs no
     // read-back); on return st_host holds the state the loop ended in.
@@ -1265,7 +1283,7 @@ class Engine {
         for (bool known = true;; known = false) {
             int r = known ? 0 : poll_state();
             if (r) return r;
-            if (st_host->done || st_host->status == ST_TIMEOUT) break;
+            if (st_host->done || timed_out()) break;
             const bool resident = use_resident();
             long long todo = resident ? RES_STEPS : chunk;
             if (nsteps > 0) {
@@ -1321,7 +1339,7 @@ class Engine {
         if (st_host->status == ST_NONFINITE)
             return fail(ESDG_E_NONFINITE, "non-finite wave speed: the solution blew up (step " +
                                               std::to_string(st_host->steps) + ")");
-        if (st_host->status == ST_TIMEOUT) return fail(ESDG_E_CUDA, "a bulk copy did not complete (bounded wait)");
+        if (timed_out()) return fail_timed_out();
         return 0;
     }
 
@@ -1359,7 +1377,7 @@ class Engine {
         if (st_host->status == ST_NONFINITE)
             return fail(ESDG_E_NONFINITE, "non-finite wave speed: the solution blew up (step " +
                                               std::to_string(st_host->steps) + ")");
-        if (st_host->status == ST_TIMEOUT) return fail(ESDG_E_CUDA, "a bulk copy did not complete (bounded wait)");
+        if (timed_out()) return fail_timed_out();
         return 0;
     }
 
@@ -1398,7 +1416,7 @@ class Engine {
         if (t_out) *t_out = st_host->t;
         if (steps_out) *steps_out = st_host->steps;
         if (st_host->status == ST_NONFINITE) return fail(ESDG_E_NONFINITE, "non-finite wave speed");
-        if (st_host->status == ST_TIMEOUT) return fail(ESDG_E_CUDA, "a bulk copy did not complete (bounded wait)");
+        if (timed_out()) return fail_timed_out();
         return 0;
     }
 
@@ -1809,6 +1827,11 @@ int esdg_resume(esdg_deviceclass* d, double* t_out, int* steps_out) {
 int esdg_debug_bulk_wait_test(esdg_deviceclass* d, long long wait_limit_cycles, int skip_tile) {
     if (!d) return ESDG_E_ARG;
     return d->eng.set_bulk_wait_test(wait_limit_cycles, skip_tile);
+}
+
+int esdg_debug_resident_wait_test(esdg_deviceclass* d, long long wait_limit_cycles) {
+    if (!d) return ESDG_E_ARG;
+    return d->eng.set_resident_wait_test(wait_limit_cycles);
 }
 
 int esdg_advance(esdg_deviceclass* d, int nsteps, double T, double* t_out, int* steps_out) {

@@ -45,7 +45,8 @@
 // shared memory holds -- hence no other size limit.
 //
 // The launch is cooperative (all CTAs resident); every wait is bounded: a
-// wait that runs out records ST_TIMEOUT and all CTAs leave.
+// wait that runs out records ST_PEER_TIMEOUT and all CTAs leave (q and the
+// step state keep what the launch started from).
 #include "esdg_resident.hpp"
 
 #include <algorithm>
@@ -455,7 +456,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_resident(const ResArgs a) {
             if (!ok) s_bad = 1;
             __syncthreads();
             if (s_bad) {  // a wait ran out: this CTA leaves, the others' waits run out too
-                if (tid == 0) atomicExch(&a.st->status, ST_TIMEOUT);
+                if (tid == 0) atomicExch(&a.st->status, ST_PEER_TIMEOUT);
                 return;
             }
             if (s == 0) {

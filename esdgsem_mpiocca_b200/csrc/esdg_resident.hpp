@@ -9,6 +9,10 @@ namespace esdg {
 
 struct ResWord;
 
+// DevState::status of a wait that ran out (ST_OK and ST_NONFINITE: kernels.cuh,
+// ST_TIMEOUT: the bulk copies, tma.cuh).
+enum : int { ST_PEER_TIMEOUT = 3 };
+
 struct ResArgs {
     int K, ne, ep;  // elements; elements per CTA (contiguous ranges) and per pass
     int fbase;      // first thread of the face warps, 0: every thread

@@ -168,6 +168,11 @@ class DeviceClass:
         copies are never issued (-1: none)."""
         self._ok(self._L.esdg_debug_bulk_wait_test(self.h, int(wait_limit_cycles), int(skip_tile)))
 
+    def debug_resident_wait_test(self, wait_limit_cycles: int):
+        """Test hook of the chip-resident loop's bounded waits: a shorter
+        wait limit (clock cycles, 0: the default)."""
+        self._ok(self._L.esdg_debug_resident_wait_test(self.h, int(wait_limit_cycles)))
+
     def set_indicator(self, mode: int, net=None):
         """Indicator of the artificial-viscosity path: 0 and 1 the modal
         sensor, the viscous terms on the active set (they are exactly zero

@@ -150,6 +150,15 @@ int esdg_resume(esdg_deviceclass* d, double* t_out, int* steps_out);
  * effect for the following launches (the step graph is captured again). */
 int esdg_debug_bulk_wait_test(esdg_deviceclass* d, long long wait_limit_cycles, int skip_tile);
 
+/* The same for the chip-resident time loop of small meshes, whose thread
+ * blocks wait for each other's traces: wait_limit_cycles sets the limit of a
+ * wait (0: the default, about 2 s).  A wait takes a thousand cycles or more,
+ * so with a limit of one the loop's first waits run out; all blocks then leave,
+ * the run returns ESDG_E_CUDA and q is as it was before the launch (of at most
+ * 1024 steps).  ESDG_E_UNSUPPORTED on a mesh whose steps run in the step
+ * graph. */
+int esdg_debug_resident_wait_test(esdg_deviceclass* d, long long wait_limit_cycles);
+
 /* Advance the resident state by up to nsteps steps (same step as
  * esdg_dg_timeloop) without any host copy of q; the device-side time and
  * step count continue from the previous call.  T is the end time. */
