@@ -341,7 +341,7 @@ def main():
                     help="ensemble workload: members solved one at a time for the plain-path rate")
     ap.add_argument("--element-variant", type=int, default=-1,
                     help="curved_lake: fix the element-kernel variant (index into the engine's variant list; "
-                         "-1: the autotuner picks), e.g. to profile one variant")
+                         "-1: the engine's choice), e.g. to profile one variant")
     args = ap.parse_args()
     if args.workload == "ensemble":
         return ensemble_bench(args)

@@ -560,11 +560,21 @@ class Engine {
     // step it may start while the kernel before it drains, which hides its
     // launch and prologue.  chained: the operation before it on the stream
     // is such a kernel too (a copy or a memset is waited for in full).
-    // Small meshes only: the launches are what a step of theirs waits for
-    // (576 elements of N = 4 with viscosity: 109.5 -> 99.8 us a step; 480,000
-    // nodes of N = 6: 2.8 % faster), while on large ones the next kernel's
-    // early blocks only take room (512x512, N = 4: no gain; 1.6 million nodes
-    // with viscosity everywhere: 8 % slower).
+    // Small meshes only: the launches are what a step of theirs waits for,
+    // while on large ones the next kernel's early blocks only take room.
+    // Measured, off against on, one variant of each mesh:
+    // viscous, few elements flagged: 8 to 12 % faster below 60,000 nodes, 3 to
+    // 9 % at 65,000 to 150,000; at 200,000 to 600,000 between 7 % faster and
+    // 3 % slower (262,144 nodes of N = 3: a tsunami 2 % slower, a dam break
+    // 1 % faster), above within 3 %.  Every element flagged: 7 % faster at
+    // 25,600, 2 % slower to equal at 100,000 to 160,000, 2 to 7 % slower above.
+    // The line lies below the sizes where that costs more than the other gains.
+    // plain, kernels with two CTAs per SM: 0 to 7 % faster at 270,000 to
+    // 600,000 nodes, 1 to 6 % at 750,000 to a million; with three or four: 1
+    // to 10 % slower at 270,000 to 600,000, above within 3 % (N = 6: 2 to 6 %
+    // slower); 512x512, N = 4: no gain.  The variant rule takes the two-CTA
+    // kernels, or the one-shot blocks, on about half of the meshes below the
+    // line and none above it (N = 1 apart).
     bool pdl_on = false, chained = false;
     bool pdl_pays() const { return (long long)K * ngl * ngl <= (AV ? 150000 : 600000); }
 

@@ -4,8 +4,9 @@
 //   face_flux  : one thread per face node gathers the two traces straight
 //                from q (wall ghost on boundary faces), evaluates the ES
 //                Riemann flux once and writes it to both elements' sides;
-//   element    : (esdg_tma.cuh, esdg_pair.cuh, esdg_rows.cuh,
-//                esdg_oneshot.cuh, whichever is fastest) flux-
+//   element    : (esdg_tma.cuh, esdg_pair.cuh or esdg_oneshot.cuh, by the
+//                rule of Engine::rule_variant; esdg_rows.cuh where a caller
+//                fixes its variants) flux-
 //                differencing volume integral, lifting of the four face
 //                fluxes, low-storage (or SSP) RK update and, on the last
 //                stage, the element wave-speed maximum for the next dt.

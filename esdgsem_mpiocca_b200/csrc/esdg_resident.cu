@@ -32,9 +32,10 @@
 //
 // Two CTAs per SM: one CTA's polls and barriers are covered by the other's
 // arithmetic.  The block bound is 256 threads (128 registers, no spills)
-// where those hold all of a CTA's nodes, else 384 (80 registers, 30 to 140
-// bytes spilled): a second pass over the nodes costs more than the spills
-// (51.8 against 59.6 us a step at 148,000 nodes of N = 4).  Where a CTA has
+// where those hold all of a CTA's nodes, else 384 (80 registers; spill stores
+// and loads of 0 and 0 bytes at N = 1, 4 to 120 and 16 to 236 at N = 2..7): a
+// second pass over the nodes costs more than the spills (51.8 against 59.6 us
+// a step at 148,000 nodes of N = 4).  Where a CTA has
 // threads to spare, whole warps take the face fluxes while the others run
 // the volume term and gather the wave-speed words.
 //
