@@ -866,7 +866,10 @@ class Engine {
     // 0.85 full, and 207 to 201 at 571,536, 0.99), on single meshes at N = 7
     // where neither pipelined kernel fills its waves (157 to 161 us at
     // 484,416), and on small plain ones that leave most of a second wave empty
-    // (47 to 50 us at 82,944 nodes, N = 3).
+    // (47 to 50 us at 82,944 nodes, N = 3).  Viscous meshes of N = 1 take
+    // them at every size (297 to 306 us in an arena of 256,056 nodes); an
+    // arena that is mostly empty does not, since their grid covers its
+    // capacity (42,456 of 2.2 million nodes live: 122 to 152 us).
     //
     // Partial-dry treatment or manufactured source: their branches cost
     // registers, and three CTAs per SM pay only on meshes larger than L2
@@ -883,7 +886,8 @@ class Engine {
         }
         constexpr int plain[7] = {0, PAIR_FIRST, 1, PAIR_FIRST + 1, 1, PAIR_FIRST + 1, PAIR_FIRST};
         constexpr int listed[7] = {0, 1, 1, PAIR_FIRST, 1, PAIR_FIRST + 1, PAIR_FIRST};
-        const int best = AV && N == 1 ? ONESHOT : (AV || arena ? listed : plain)[N - 1];
+        const bool live = !arena || 2 * (long long)Kl > K;
+        const int best = AV && N == 1 && live ? ONESHOT : (AV || arena ? listed : plain)[N - 1];
         if (!pdl_pays() || N == 1) return best;
         const int big = AV ? 1 : best;
         auto waves = [&](int v, int ne) { return (double)((Kl + ne - 1) / ne) / (std::max(1, tma_ctas[v]) * sm_count()); };

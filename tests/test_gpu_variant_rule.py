@@ -12,6 +12,7 @@ import pytest
 
 from esdgsem_mpiocca_b200 import host, problems
 from esdgsem_mpiocca_b200.deviceclass import Solver
+from esdgsem_mpiocca_b200.ensemble import Ensemble
 
 pytestmark = pytest.mark.gpu
 
@@ -83,3 +84,17 @@ def test_queries_only_read():
     np.testing.assert_array_equal(out[0][2], out[1][2])
     np.testing.assert_array_equal(out[0][3], out[1][3])
     assert seen and all(v is None or v == final for v, _ in seen)
+
+
+def test_mostly_empty_arena_takes_no_one_shot_blocks():
+    """Their grid covers the arena's capacity."""
+    pr = problems.dam_break(N=1, nel=20)
+    for slack, want in ((1.0, 7), (40.0, TWO_CTAS)):
+        ens = Ensemble.for_problems([pr], slack=slack)
+        try:
+            i = ens.add(pr, T=1e9, max_steps=3)
+            ens.advance(3)
+            assert ens.element_variants()["chosen"] == want
+            assert np.isfinite(ens.q(i)).all()
+        finally:
+            ens.close()
